@@ -1,0 +1,7 @@
+// psg_chip2d_f32.cu -- the on-chip 2D integrator's FP32 kernels (psg_chip2d_run.cuh)
+#define PSG_CHIP2D_INSTANTIATE
+#include "psg_chip2d_run.cuh"
+
+namespace psg {
+PSG_CHIP2D_TEMPLATES(float)
+}  // namespace psg

@@ -1,7 +1,8 @@
-// psg_ns2d.cu -- 2D vorticity RK4/CN step as one persistent CTA per instance
-// (kernel body in psg_ns2d.cuh).  Any number of instances of any supported
-// size run in one launch: blocks take instances from a work counter, largest
-// first as ordered by the host.
+// psg_ns2d.cu -- batches of independent 2D vorticity RK4/CN runs: every instance
+// is integrated on chip by a thread-block cluster of its own (psg_chip2d.cuh).
+// Any number of instances of any supported size run in one graph launch, one
+// kernel per size present, largest size first; the hardware starts the clusters
+// in order of their expected length as room becomes free.
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -10,39 +11,31 @@
 #include <type_traits>
 #include <vector>
 
-#include "psg_ns2d.cuh"
+#include "psg_chip2d_run.cuh"
 #include "psgpu_internal.h"
 
 namespace psg {
 
-template <typename T>
-struct Twiddles2D {
-  const cpx<T>* t[5];  // n = 16, 32, 64, 128, 256
-  int pk = 0;          // bit q: size class q runs the packed transforms (FP32)
-};
-
-template <typename T, int NN, bool HASPK>
-__device__ __forceinline__ void rhs2d_run(const Inst2D<T>& I, const cpx<T>* tw, cpx<T>* smem,
-                                          bool pk) {
-  if constexpr (sizeof(T) == 4 && HASPK) {
-    if (pk) {
-      Rhs2D<T, NN, 1>::run(I, tw, smem);
-      return;
-    }
-  }
-  Rhs2D<T, NN>::run(I, tw, smem);
-}
-
-// block sizes of the persistent kernel the autotuner chooses from
+// the size class of a grid: n = 16 << class
+constexpr int kClasses = 5;
+constexpr int size_class(int n) { return n == 16 ? 0 : n == 32 ? 1 : n == 64 ? 2 : n == 128 ? 3 : n == 256 ? 4 : -1; }
+// threads per block the autotuner chooses from (at most; a cluster's blocks take
+// no more than they have lines for)
 constexpr int kBlock2D[3] = {128, 256, 512};
 
-// HASPK: the packed transform schedules are compiled in (a schedule with no
-// packed size class launches the build without them, whose registers are
-// those of the scalar transforms alone)
-template <typename T, int NT, bool HASPK = false>
-__global__ void __launch_bounds__(NT)
-ns2d_persistent(const Inst2D<T>* __restrict__ insts, int ninst, int* __restrict__ next,
-                Twiddles2D<T> tws) {
+// One block per instance with the row scratch in global memory (Rhs2D), for large
+// FP64 batches of 128^2 and 256^2: their lines in FP64 need 4 and 16 blocks'
+// shared memory, so that only 33 and 7 clusters fit the device at once, and once
+// every SM has an instance of its own the cluster barriers cost more than the L2
+// traffic: 148 instances of 128^2 202 against 239 us a step, of 256^2 940
+// against 1303 (in FP32 the chip integrator is the faster at every count).
+// Instances are claimed from a counter.
+constexpr int kGlobalMin[kClasses] = {0, 0, 0, 133, 97};  // instances from which it is used (0: never)
+constexpr int kGlobalThreads = 512;
+template <typename T>
+__global__ void __launch_bounds__(kGlobalThreads)
+ns2d_global(const Inst2D<T>* __restrict__ insts, int ninst, int* __restrict__ next,
+            const cpx<T>* __restrict__ tw128, const cpx<T>* __restrict__ tw256) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cpx<T>* smem = reinterpret_cast<cpx<T>*>(smem_raw);
   __shared__ int s_idx;
@@ -53,13 +46,8 @@ ns2d_persistent(const Inst2D<T>* __restrict__ insts, int ninst, int* __restrict_
     const int i = s_idx;
     if (i >= ninst) break;
     const Inst2D<T> I = insts[i];
-    switch (I.n) {
-      case 16: rhs2d_run<T, 16, HASPK>(I, tws.t[0], smem, tws.pk & 1); break;
-      case 32: rhs2d_run<T, 32, HASPK>(I, tws.t[1], smem, tws.pk & 2); break;
-      case 64: rhs2d_run<T, 64, HASPK>(I, tws.t[2], smem, tws.pk & 4); break;
-      case 128: rhs2d_run<T, 128, HASPK>(I, tws.t[3], smem, tws.pk & 8); break;
-      default: rhs2d_run<T, 256, HASPK>(I, tws.t[4], smem, tws.pk & 16); break;
-    }
+    if (I.n == 128) Rhs2D<T, 128>::run(I, tw128, smem);
+    else Rhs2D<T, 256>::run(I, tw256, smem);
   }
 }
 
@@ -109,39 +97,51 @@ struct Batch2D final : Batch2DBase {
   int ninst = 0;
   std::vector<int> sizes;
   std::vector<long> offs;     // state offset of each instance (complex words)
-  std::vector<long> woffs;    // work offset
+  std::vector<long> woffs;    // offset of the stage sums
   cpx<T>* pool = nullptr;
   cpx<T>* twp = nullptr;
-  Inst2D<T>* d_insts = nullptr;
-  int* d_next = nullptr;
+  ChipInst<T>* d_insts = nullptr;
   double2* staging = nullptr;
   long staging_len = 0;
   cudaStream_t stream = 0;
   long launches = 0;
   std::vector<int> order;     // instances sorted by cost, largest first
-  size_t smem_v[3] = {0, 0, 0};  // dynamic shared memory per block-size variant
-  int grid_v[3] = {0, 0, 0};     // resident blocks per variant (0: does not fit)
-  int grid_pk[3] = {0, 0, 0};    // the same for the build with packed schedules
-  int variant = 1;               // 256 threads unless the autotuner picks another
+  int count[kClasses] = {0, 0, 0, 0, 0};  // instances of each size
+  // per size, block-size variant and transform schedule (scalar, packed): the
+  // kernel and its launch shape; fn == nullptr where it does not fit
+  ChipPlan plan[kClasses][3][2];
+  // FP64 sizes run by ns2d_global: their instances, counter, blocks and scratch
+  bool global[kClasses] = {false, false, false, false, false};
+  int nglobal = 0, global_grid = 0;
+  size_t global_smem = 0;
+  Inst2D<T>* d_global = nullptr;
+  int* d_next = nullptr;
+  int variant = 1;               // up to 256 threads unless the autotuner picks another
   float tune_ms[3] = {-1.f, -1.f, -1.f};
   // transform schedule per size class (n = 16 .. 256): bit q packed f32x2
   // transforms (FP32), chosen by the autotuner; sched_ms[q][0 / 1] the timing of
   // the batch with class q scalar / packed (-1: class absent or not timed)
   int pk_mask = 0;
   float sched_ms[5][2] = {{-1.f, -1.f}, {-1.f, -1.f}, {-1.f, -1.f}, {-1.f, -1.f}, {-1.f, -1.f}};
-  int gexec_pk = -1;
   long state_words = 0;          // states (+ carried errors) of all instances
   bool params_set = false;
-  // the persistent launch as a CUDA graph: reset the work counter, launch
+  // the launch as a CUDA graph, one kernel per size on branches of their own
   cudaGraphExec_t gexec = nullptr;
-  int gexec_variant = -1;
-  cudaStream_t cap = nullptr;
+  int gexec_variant = -1, gexec_pk = -1;
+  cudaStream_t cap = nullptr, side[kClasses] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  cudaEvent_t ev_fork = nullptr, ev_join[kClasses] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 
   ~Batch2D() override {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (cap) cudaStreamDestroy(cap);
+    for (int q = 0; q < kClasses; ++q) {
+      if (side[q]) cudaStreamDestroy(side[q]);
+      if (ev_join[q]) cudaEventDestroy(ev_join[q]);
+    }
+    if (ev_fork) cudaEventDestroy(ev_fork);
     if (pool) cudaFree(pool);
     if (d_insts) cudaFree(d_insts);
+    if (d_global) cudaFree(d_global);
     if (d_next) cudaFree(d_next);
     if (staging) cudaFree(staging);
   }
@@ -149,147 +149,162 @@ struct Batch2D final : Batch2DBase {
   int init(int n_, const int* sizes_) {
     ninst = n_;
     sizes.assign(sizes_, sizes_ + n_);
-    long total = 0, work = 0, maxk = 0;
+    long total = 0, sums = 0, maxk = 0;
     for (int i = 0; i < ninst; ++i) {
-      const int n = sizes[i];
-      if (!(n == 16 || n == 32 || n == 64 || n == 128 || n == 256)) {
+      const int n = sizes[i], q = size_class(n);
+      if (q < 0) {
         psg_set_error("2D grid size %d unsupported (powers of two 16..256)", n);
         return PSG_ERR_UNSUPPORTED;
       }
+      ++count[q];
       offs.push_back(total);
-      total += (std::is_same<T, float>::value ? 6L : 5L) * nkt2(n);
+      total += (std::is_same<T, float>::value ? 2L : 1L) * nkt2(n);
       maxk = std::max<long>(maxk, nkt2(n));
     }
     state_words = total;
+    for (int q = 0; q < kClasses; ++q) {
+      global[q] = sizeof(T) == 8 && kGlobalMin[q] && count[q] >= kGlobalMin[q];
+      if (global[q]) nglobal += count[q];
+    }
+    // the sums of the stage increments, for sizes whose state arrays stay outside
+    // shared memory; the stage registers and rows of the global-memory kernel
     for (int i = 0; i < ninst; ++i) {
-      woffs.push_back(total + work);
-      work += 3L * sizes[i] * (sizes[i] / 3 + 1);
+      woffs.push_back(total + sums);
+      const long nk = nkt2(sizes[i]);
+      sums += global[size_class(sizes[i])] ? 4 * nk + 3L * sizes[i] * (sizes[i] / 3 + 1) : nk;
     }
     const long twlen = 2 * (16 + 32 + 64 + 128 + 256);
-    PSG_CUDA_TRY(cudaMalloc(&pool, sizeof(cpx<T>) * (total + work + twlen)));
-    PSG_CUDA_TRY(cudaMemset(pool, 0, sizeof(cpx<T>) * (total + work + twlen)));
-    twp = pool + total + work;
+    PSG_CUDA_TRY(cudaMalloc(&pool, sizeof(cpx<T>) * (total + sums + twlen)));
+    PSG_CUDA_TRY(cudaMemset(pool, 0, sizeof(cpx<T>) * (total + sums + twlen)));
+    twp = pool + total + sums;
     std::vector<cpx<T>> h(twlen);
     tables2d(h.data());
     PSG_CUDA_TRY(cudaMemcpy(twp, h.data(), sizeof(cpx<T>) * twlen, cudaMemcpyHostToDevice));
-    PSG_CUDA_TRY(cudaMalloc(&d_insts, sizeof(Inst2D<T>) * ninst));
-    PSG_CUDA_TRY(cudaMalloc(&d_next, sizeof(int)));
+    PSG_CUDA_TRY(cudaMalloc(&d_insts, sizeof(ChipInst<T>) * ninst));
+    if (nglobal) {
+      PSG_CUDA_TRY(cudaMalloc(&d_global, sizeof(Inst2D<T>) * nglobal));
+      PSG_CUDA_TRY(cudaMalloc(&d_next, sizeof(int)));
+    }
     staging_len = maxk;
     PSG_CUDA_TRY(cudaMalloc(&staging, sizeof(double2) * staging_len));
     order.resize(ninst);
     for (int i = 0; i < ninst; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sizes[a] > sizes[b]; });
-    int maxn = 16;
-    for (int n : sizes) maxn = std::max(maxn, n);
-    int g = 4, sm = 0;
-    switch (maxn) {
-      case 16: g = LineFFT<16, 1, T>::G; sm = LineFFT<16, 1, T>::SMEM; break;
-      case 32: g = LineFFT<32, 1, T>::G; sm = LineFFT<32, 1, T>::SMEM; break;
-      case 64: g = LineFFT<64, 1, T>::G; sm = LineFFT<64, 1, T>::SMEM; break;
-      case 128: g = LineFFT<128, 1, T>::G; sm = LineFFT<128, 1, T>::SMEM; break;
-      default: g = LineFFT<256, 1, T>::G; sm = LineFFT<256, 1, T>::SMEM; break;
-    }
-    // exchange space for the densest packing of groups over all sizes present
-    size_t worst = 0;
-    for (int n : sizes) {
-      int gg = 4, ss = 0;
-      switch (n) {
-        case 16: gg = LineFFT<16, 1, T>::G; ss = LineFFT<16, 1, T>::SMEM; break;
-        case 32: gg = LineFFT<32, 1, T>::G; ss = LineFFT<32, 1, T>::SMEM; break;
-        case 64: gg = LineFFT<64, 1, T>::G; ss = LineFFT<64, 1, T>::SMEM; break;
-        case 128: gg = LineFFT<128, 1, T>::G; ss = LineFFT<128, 1, T>::SMEM; break;
-        default: gg = LineFFT<256, 1, T>::G; ss = LineFFT<256, 1, T>::SMEM; break;
-      }
-      for (int v = 0; v < 3; ++v)
-        smem_v[v] = std::max(smem_v[v], sizeof(cpx<T>) * (size_t)(2 * n + (kBlock2D[v] / gg) * ss));
-    }
-    (void)g; (void)sm;
-    int dev = 0, nsm = 148, big = 0;
-    PSG_CUDA_TRY(cudaGetDevice(&dev));
-    PSG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    PSG_CUDA_TRY(cudaDeviceGetAttribute(&big, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    for (int v = 0; v < 3; ++v) {
-      const void* k = kernel(v);
-      grid_v[v] = 0;
-      if (smem_v[v] + 1024 > (size_t)big) continue;
-      PSG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem_v[v]));
-      int per_sm = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBlock2D[v], smem_v[v]);
-      grid_v[v] = std::max(0, std::min(ninst, nsm * per_sm));
-      grid_pk[v] = 0;
-      if constexpr (sizeof(T) == 4) {
-        const void* kp = kernel_pk(v);
-        PSG_CUDA_TRY(cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem_v[v]));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kp, kBlock2D[v], smem_v[v]);
-        grid_pk[v] = std::max(0, std::min(ninst, nsm * per_sm));
-      }
-    }
-    if (!grid_v[variant]) {
-      variant = -1;
-      for (int v = 0; v < 3 && variant < 0; ++v)
-        if (grid_v[v]) variant = v;
-      if (variant < 0) {
-        psg_set_error("2D batch: no block size fits this device");
-        return PSG_ERR_UNSUPPORTED;
-      }
-    }
+    if (int rc = choose_plans()) return rc;
     PSG_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     return PSG_OK;
   }
 
-  static const void* kernel(int v) {
-    switch (v) {
-      case 0: return (const void*)ns2d_persistent<T, 128>;
-      case 1: return (const void*)ns2d_persistent<T, 256>;
-      default: return (const void*)ns2d_persistent<T, 512>;
-    }
-  }
-  static const void* kernel_pk(int v) {
-    switch (v) {
-      case 0: return (const void*)ns2d_persistent<T, 128, true>;
-      case 1: return (const void*)ns2d_persistent<T, 256, true>;
-      default: return (const void*)ns2d_persistent<T, 512, true>;
-    }
-  }
-
-  Twiddles2D<T> twiddles() const {
-    Twiddles2D<T> tws;
-    long o = 0;
-    for (int q = 0, n = 16; q < 5; ++q, n *= 2) { tws.t[q] = twp + o; o += 2 * n; }
-    tws.pk = pk_mask;
-    return tws;
-  }
-
-  void launch_kernel(int v, cudaStream_t st) {
-    const Twiddles2D<T> tws = twiddles();
-    if constexpr (sizeof(T) == 4) {
-      if (tws.pk) {
-      switch (v) {
-        case 0: ns2d_persistent<T, 128, true><<<grid_pk[0], 128, smem_v[0], st>>>(d_insts, ninst, d_next, tws); break;
-        case 1: ns2d_persistent<T, 256, true><<<grid_pk[1], 256, smem_v[1], st>>>(d_insts, ninst, d_next, tws); break;
-        default: ns2d_persistent<T, 512, true><<<grid_pk[2], 512, smem_v[2], st>>>(d_insts, ninst, d_next, tws); break;
-      }
-      return;
+  // Cluster size of every size present.  A batch that leaves SMs idle spreads each
+  // instance over as many blocks as there is room for, the largest grids first; a
+  // batch that fills the device takes the smallest cluster that holds the grid
+  // (fewest barriers and the least traffic between blocks per step).  One 128^2
+  // FP64 run: 57 us a step on 4 blocks, 37 on 8, 30 on 16; 400 of them: see DESIGN.
+  int choose_plans() {
+    int dev = 0, nsm = 148;
+    PSG_CUDA_TRY(cudaGetDevice(&dev));
+    PSG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    int cs[kClasses] = {0, 0, 0, 0, 0};
+    long blocks = nglobal;
+    ChipPlan p;
+    if constexpr (sizeof(T) == 8) {
+      if (nglobal) {
+        const size_t a = kGlobalThreads / LineFFT<128, 1, T>::G * LineFFT<128, 1, T>::SMEM + 2 * 128;
+        const size_t b = kGlobalThreads / LineFFT<256, 1, T>::G * LineFFT<256, 1, T>::SMEM + 2 * 256;
+        global_smem = sizeof(cpx<T>) * std::max(global[3] ? a : 0, global[4] ? b : 0);
+        int occ = 0;
+        PSG_CUDA_TRY(cudaFuncSetAttribute(ns2d_global<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)global_smem));
+        PSG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ns2d_global<T>, kGlobalThreads,
+                                                                   global_smem));
+        global_grid = std::min(nglobal, nsm * std::max(occ, 1));
       }
     }
-    switch (v) {
-      case 0: ns2d_persistent<T, 128><<<grid_v[0], 128, smem_v[0], st>>>(d_insts, ninst, d_next, tws); break;
-      case 1: ns2d_persistent<T, 256><<<grid_v[1], 256, smem_v[1], st>>>(d_insts, ninst, d_next, tws); break;
-      default: ns2d_persistent<T, 512><<<grid_v[2], 512, smem_v[2], st>>>(d_insts, ninst, d_next, tws); break;
+    for (int q = 0; q < kClasses; ++q) {
+      if (!count[q] || global[q]) continue;
+      for (int c = 1; c <= 16 && !cs[q]; c *= 2)
+        if (chip2d_plan<T>(16 << q, c, CHIP_STEP, 0, 256, &p)) cs[q] = c;
+      if (!cs[q]) {
+        psg_set_error("2D batch: no kernel for grid %d fits this device", 16 << q);
+        return PSG_ERR_UNSUPPORTED;
+      }
+      blocks += (long)count[q] * cs[q];
     }
+    for (int q = kClasses - 1; q >= 0; --q) {
+      if (!count[q] || global[q]) continue;
+      for (int c = 2 * cs[q]; c <= 16; c *= 2) {
+        // a cluster lies in one GPC: of 16 blocks (one per SM) 7 fit the device, of
+        // 8 15, of 4 33
+        const int room = c == 16 ? 7 * 16 : c == 8 ? 15 * 8 : c == 4 ? 33 * 4 : nsm;
+        if (blocks + (long)count[q] * (c - cs[q]) > std::min(room, nsm)) break;
+        if (!chip2d_plan<T>(16 << q, c, CHIP_STEP, 0, 256, &p)) continue;
+        blocks += (long)count[q] * (c - cs[q]);
+        cs[q] = c;
+      }
+    }
+    for (int q = 0; q < kClasses; ++q)
+      for (int v = 0; v < 3 && count[q] && !global[q]; ++v)
+        for (int k = 0; k < (sizeof(T) == 4 ? 2 : 1); ++k)
+          chip2d_plan<T>(16 << q, cs[q], CHIP_STEP, k, kBlock2D[v], &plan[q][v][k]);
+    return PSG_OK;
   }
 
-  // (re)build the graph of one persistent launch for the current variant
+  const ChipPlan& plan_of(int q, int v) const { return plan[q][v][(pk_mask >> q) & 1]; }
+  // every size present has a kernel of block-size variant v under schedule `mask`
+  bool fits(int v, int mask) const {
+    for (int q = 0; q < kClasses; ++q)
+      if (count[q] && !global[q] && !plan[q][v][(mask >> q) & 1].fn) return false;
+    return true;
+  }
+
+  const cpx<T>* twiddles(int q) const { return twp + 2 * (16 * ((1 << q) - 1)); }
+
+  // one kernel per size present, on streams of their own when there are several
+  int launch_kernel(int v, cudaStream_t st) {
+    int present = 0;
+    for (int q = 0; q < kClasses; ++q) present += count[q] > 0;
+    if (present > 1 && !ev_fork) {
+      for (int q = 0; q < kClasses; ++q) {
+        PSG_CUDA_TRY(cudaStreamCreateWithFlags(&side[q], cudaStreamNonBlocking));
+        PSG_CUDA_TRY(cudaEventCreateWithFlags(&ev_join[q], cudaEventDisableTiming));
+      }
+      PSG_CUDA_TRY(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+    }
+    if (present > 1) PSG_CUDA_TRY(cudaEventRecord(ev_fork, st));
+    int off = 0;
+    bool global_sent = false;
+    for (int q = kClasses - 1; q >= 0; --q) {
+      if (!count[q]) continue;
+      cudaStream_t s = present > 1 ? side[q] : st;
+      if (present > 1) PSG_CUDA_TRY(cudaStreamWaitEvent(s, ev_fork, 0));
+      if (global[q]) {  // all such sizes in the first one's launch
+        if constexpr (sizeof(T) == 8)
+          if (!global_sent) {
+            global_sent = true;
+            PSG_CUDA_TRY(cudaMemsetAsync(d_next, 0, sizeof(int), s));
+            ns2d_global<T><<<global_grid, kGlobalThreads, global_smem, s>>>(d_global, nglobal, d_next,
+                                                                          twiddles(3), twiddles(4));
+            PSG_CUDA_TRY(cudaGetLastError());
+          }
+      } else PSG_CUDA_TRY(chip2d_launch<T>(plan_of(q, v), d_insts + off, count[q], twiddles(q), s));
+      if (present > 1) {
+        PSG_CUDA_TRY(cudaEventRecord(ev_join[q], s));
+        PSG_CUDA_TRY(cudaStreamWaitEvent(st, ev_join[q], 0));
+      }
+      off += count[q];
+    }
+    return PSG_OK;
+  }
+
+  // (re)build the graph of one launch for the current variant and schedule
   int build_graph() {
     if (gexec && gexec_variant == variant && gexec_pk == pk_mask) return PSG_OK;
     if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
     cudaGraph_t graph = nullptr;
     PSG_CUDA_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(d_next, 0, sizeof(int), cap);
-    launch_kernel(variant, cap);
+    const int rc = launch_kernel(variant, cap);
     cudaError_t e = cudaStreamEndCapture(cap, &graph);
+    if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
     if (e != cudaSuccess) { psg_set_error("graph capture: %s", cudaGetErrorString(e)); return PSG_ERR_CUDA; }
     e = cudaGraphInstantiate(&gexec, graph, 0);
     cudaGraphDestroy(graph);
@@ -302,7 +317,7 @@ struct Batch2D final : Batch2DBase {
   // carried rounding error of instance i's state (FP32 engine), or null
   cpx<T>* comp(int i) {
     if (!std::is_same<T, float>::value) return nullptr;
-    return pool + offs[i] + 5L * nkt2(sizes[i]);
+    return pool + offs[i] + nkt2(sizes[i]);
   }
 
   int upload(int i, const double* Z) override {
@@ -345,25 +360,21 @@ struct Batch2D final : Batch2DBase {
   // transforms), one class at a time, keeping the faster
   int autotune(int* v_out, float* ms) override {
     if (!params_set) { psg_set_error("2D batch: parameters not set"); return PSG_ERR_STATE; }
-    std::vector<Inst2D<T>> h(hparams), shortp(hparams);
+    std::vector<ChipInst<T>> h(hparams), shortp(hparams);
     for (auto& I : shortp) I.nsteps = std::min(I.nsteps, 2);
     cpx<T>* save = nullptr;
     PSG_CUDA_TRY(cudaMalloc(&save, sizeof(cpx<T>) * state_words));
     PSG_CUDA_TRY(cudaMemcpyAsync(save, pool, sizeof(cpx<T>) * state_words, cudaMemcpyDeviceToDevice, stream));
-    PSG_CUDA_TRY(cudaMemcpyAsync(d_insts, shortp.data(), sizeof(Inst2D<T>) * ninst,
-                                 cudaMemcpyHostToDevice, stream));
+    if (int rc = push_insts(shortp)) { cudaFree(save); return rc; }
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     // ms per launch of the short run with block-size variant v and the current schedule
     auto time_v = [&](int v, float* out) -> int {
-      cudaMemsetAsync(d_next, 0, sizeof(int), stream);
-      launch_kernel(v, stream);
+      if (int rc = launch_kernel(v, stream)) return rc;
       cudaEventRecord(a, stream);
-      for (int r = 0; r < 3; ++r) {
-        cudaMemsetAsync(d_next, 0, sizeof(int), stream);
-        launch_kernel(v, stream);
-      }
+      for (int r = 0; r < 3; ++r)
+        if (int rc = launch_kernel(v, stream)) return rc;
       cudaEventRecord(b, stream);
       launches += 4;
       cudaError_t e = cudaEventSynchronize(b);
@@ -378,7 +389,7 @@ struct Batch2D final : Batch2DBase {
     int pick = variant;
     for (int v = 0; v < 3 && !rc; ++v) {
       tune_ms[v] = -1.f;
-      if (!grid_v[v]) continue;
+      if (!fits(v, pk_mask)) continue;
       rc = time_v(v, &tune_ms[v]);
       if (!rc && tune_ms[v] < best) { best = tune_ms[v]; pick = v; }
     }
@@ -388,8 +399,8 @@ struct Batch2D final : Batch2DBase {
       for (int n : sizes)
         for (int q = 0; q < 5; ++q)
           if (n == (16 << q)) present |= 1 << q;
-      for (int q = 0; q < 5 && !rc && grid_pk[pick] > 0; ++q) {
-        if (!(present & (1 << q))) continue;
+      for (int q = 0; q < 5 && !rc; ++q) {
+        if (!(present & (1 << q)) || !plan[q][pick][1].fn) continue;
         for (int p = 0; p < 2 && !rc; ++p) {
           pk_mask = p ? (pk_mask | (1 << q)) : (pk_mask & ~(1 << q));
           rc = time_v(pick, &sched_ms[q][p]);
@@ -402,9 +413,7 @@ struct Batch2D final : Batch2DBase {
     cudaEventDestroy(b);
     if (rc) { cudaFree(save); return rc; }
     PSG_CUDA_TRY(cudaMemcpyAsync(pool, save, sizeof(cpx<T>) * state_words, cudaMemcpyDeviceToDevice, stream));
-    PSG_CUDA_TRY(cudaMemcpyAsync(d_insts, h.data(), sizeof(Inst2D<T>) * ninst,
-                                 cudaMemcpyHostToDevice, stream));
-    PSG_CUDA_TRY(cudaStreamSynchronize(stream));
+    if (int rc2 = push_insts(h)) { cudaFree(save); return rc2; }
     cudaFree(save);
     variant = pick;
     if (v_out) *v_out = variant;
@@ -416,7 +425,7 @@ struct Batch2D final : Batch2DBase {
     int m = 0;
     for (int q = 0; q < 5; ++q)
       if (pk[q]) m |= 1 << q;
-    if (m && (sizeof(T) != 4 || !grid_pk[variant])) {
+    if (m && (sizeof(T) != 4 || !fits(variant, m))) {
       psg_set_error("packed transforms need an FP32 batch whose packed build fits");
       return PSG_ERR_UNSUPPORTED;
     }
@@ -432,26 +441,48 @@ struct Batch2D final : Batch2DBase {
     return PSG_OK;
   }
 
-  std::vector<Inst2D<T>> hparams;
+  std::vector<ChipInst<T>> hparams;
 
   int set_params(const double* nu, const double* dt, const int* nsteps) override {
-    std::vector<Inst2D<T>> h(ninst);
+    // largest grid first (the sizes' kernels take runs of the list), longest run first
+    std::vector<int> ord(order);
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
+      return sizes[a] != sizes[b] ? sizes[a] > sizes[b] : nsteps[a] > nsteps[b];
+    });
+    std::vector<ChipInst<T>> h(ninst);
     for (int j = 0; j < ninst; ++j) {
-      const int i = order[j];
-      const long nk = nkt2(sizes[i]);
-      Inst2D<T>& I = h[j];
-      I.n = sizes[i]; I.nsteps = nsteps[i]; I.nu = (T)nu[i]; I.dt = (T)dt[i];
-      cpx<T>* b = pool + offs[i];
-      I.Z = b; I.Z0 = b + nk; I.Z1 = b + 2 * nk; I.Z2 = b + 3 * nk; I.Z3 = b + 4 * nk;
-      I.work = pool + woffs[i];
-      I.ZC = comp(i);
+      const int i = ord[j];
+      ChipInst<T>& I = h[j];
+      I.nsteps = nsteps[i]; I.mode = 0; I.nu = (T)nu[i]; I.dt = (T)dt[i];
+      I.Z = pool + offs[i]; I.D = nullptr; I.ZC = comp(i); I.acc = pool + woffs[i];
     }
-    PSG_CUDA_TRY(cudaMemcpyAsync(d_insts, h.data(), sizeof(Inst2D<T>) * ninst,
-                                 cudaMemcpyHostToDevice, stream));
-    // the copy reads pageable host memory: finish it before h goes away
-    PSG_CUDA_TRY(cudaStreamSynchronize(stream));
+    hsizes.resize(ninst);
+    for (int j = 0; j < ninst; ++j) hsizes[j] = sizes[ord[j]];
+    if (int rc = push_insts(h)) return rc;
     hparams = h;
     params_set = true;
+    return PSG_OK;
+  }
+
+  std::vector<int> hsizes;  // grid sizes in the order of hparams
+  // the instance descriptors to the device (waits for the copies)
+  int push_insts(const std::vector<ChipInst<T>>& h) {
+    PSG_CUDA_TRY(cudaMemcpyAsync(d_insts, h.data(), sizeof(ChipInst<T>) * ninst,
+                                 cudaMemcpyHostToDevice, stream));
+    std::vector<Inst2D<T>> g;
+    for (int j = 0; j < ninst; ++j) {
+      const int n = hsizes[j];
+      if (!global[size_class(n)]) continue;
+      const long nk = nkt2(n);
+      cpx<T>* b = h[j].acc;
+      g.push_back(Inst2D<T>{n, h[j].nsteps, h[j].nu, h[j].dt, h[j].Z, b, b + nk, b + 2 * nk, b + 3 * nk,
+                            b + 4 * nk, h[j].ZC});
+    }
+    if (!g.empty())
+      PSG_CUDA_TRY(cudaMemcpyAsync(d_global, g.data(), sizeof(Inst2D<T>) * g.size(),
+                                   cudaMemcpyHostToDevice, stream));
+    // the copies read pageable host memory: finish them before it goes away
+    PSG_CUDA_TRY(cudaStreamSynchronize(stream));
     return PSG_OK;
   }
 
