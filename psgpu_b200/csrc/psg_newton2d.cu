@@ -27,6 +27,7 @@
 #include <chrono>
 #include <vector>
 
+#include "psg_chip2d_run.cuh"
 #include "psg_tan2d_run.cuh"
 
 namespace psg {
@@ -327,7 +328,7 @@ struct Upo2D {
   bool prof = false;
   double t_int[4] = {0, 0, 0, 0}, t_svd = 0, t_solve = 0;
   // blocks per instance (a cluster) when the batch leaves room: at most this many
-  int cluster_max = 4;
+  int cluster_max = 16;
   // side streams and events of integrations split over several launches
   cudaStream_t side[3] = {nullptr, nullptr, nullptr};
   cudaEvent_t ev_fork = nullptr, ev_join[3] = {nullptr, nullptr, nullptr};
@@ -414,7 +415,8 @@ struct Upo2D {
     for (int g = 0; g < ng; ++g)
       for (int j = 0; j <= kmax; ++j) qp[(size_t)g * (kmax + 1) + j] = G[g].q[j];
     PSG_CUDA_TRY(cudaMemcpy(d_qptr, qp.data(), sizeof(C2*) * qp.size(), cudaMemcpyHostToDevice));
-    // PSG_UPO_CLUSTER: the largest cluster an integration may use (1, 2 or 4)
+    // PSG_UPO_CLUSTER: the largest cluster an integration may use (1 .. 16; a grid
+    // that needs more blocks than that takes the fewest it fits in)
     if (const char* e = getenv("PSG_UPO_CLUSTER")) cluster_max = atoi(e);
     return PSG_OK;
   }
@@ -463,6 +465,33 @@ struct Upo2D {
     return PSG_OK;
   }
 
+  // The on-chip integrator's launch shape for `ni` integrations of `kind`: the
+  // cluster size and threads with the least expected time, waves of resident
+  // clusters times the time of one (a step of one 128^2 FP64 tangent: 62 us on 8
+  // blocks, 45 on 16; of a 64^2 one 75 us on one block, 33 on 4).  False where no
+  // kernel holds the grid (256^2 FP64 tangents: the global-memory integrator), and
+  // for grids up to 32^2, where there is the least to gain (19 against 33 us a
+  // step) and the continuation's corrector follows its FP64 restatement to 1e-7 of
+  // a residual whose rounding noise the Newton steps amplify by 1e9: those keep
+  // the integrator whose rounding that agreement was established with.
+  template <typename T>
+  bool chip_shape(int kind, int ni, ChipPlan* out) {
+    if (n <= 32) return false;
+    static const double rel[5] = {1.0, 0.65, 0.42, 0.27, 0.21};  // 1, 2, 4, 8, 16 blocks
+    double best = 0.0;
+    ChipPlan p;
+    for (int c = 0; c < 5; ++c) {
+      if ((1 << c) > cluster_max && best > 0.0) break;
+      for (int th = 128; th <= 256; th *= 2) {
+        if (!chip2d_plan<T>(n, 1 << c, kind, 0, th, &p)) continue;
+        const double waves = (ni + p.resident - 1) / p.resident;
+        const double cost = waves * rel[c] * (p.threads <= 128 ? 1.1 : 1.0);
+        if (best == 0.0 || cost < best) { best = cost; *out = p; }
+      }
+    }
+    return best > 0.0;
+  }
+
   template <typename T>
   int integrate_t(const std::vector<IntReq>& reqs, IntPlan<T>& plan) {
     constexpr bool is32 = sizeof(T) == 4;
@@ -498,6 +527,27 @@ struct Upo2D {
     }
     if (is32)
       if (int rc = convert(in_jobs, true)) return rc;
+    const int kind = reqs[0].mode == 0 ? CHIP_TANGENT : CHIP_BASE;
+    bool same = true;
+    for (const IntReq& r : reqs) same = same && r.mode == reqs[0].mode;
+    ChipPlan cp;
+    if (same && chip_shape<T>(kind, (int)h.size(), &cp)) {
+      // one cluster per guess, the longest integrations first
+      std::stable_sort(h.begin(), h.end(), [](const InstTan2D<T>& a, const InstTan2D<T>& b) {
+        return a.nsteps > b.nsteps;
+      });
+      std::vector<ChipInst<T>> ci;
+      for (const InstTan2D<T>& I : h)
+        ci.push_back(ChipInst<T>{I.nsteps, I.mode, I.nu, I.dt, I.Z, I.D, nullptr, I.Z1});
+      PSG_CUDA_TRY(cudaMemcpyAsync(plan.d_chip, ci.data(), sizeof(ChipInst<T>) * ci.size(),
+                                   cudaMemcpyHostToDevice, stream));
+      PSG_CUDA_TRY(chip2d_launch<T>(cp, plan.d_chip, (int)ci.size(), plan.tw, stream));
+      ++launches;
+      if (is32)
+        if (int rc = convert(out_jobs, false)) return rc;
+      integrations += (long)ci.size();
+      return PSG_OK;
+    }
     // blocks per guess: every guess starts with one; while blocks are left
     // (the resident capacity of the device at the integrator's registers), the
     // guess that would finish last moves to a cluster of two, then four.

@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "psg_chip2d.cuh"
 #include "psg_tan2d.cuh"
 #include "psgpu_internal.h"
 
@@ -144,6 +145,7 @@ template <typename T>
 struct IntPlan {
   cpx<T>* tw = nullptr;
   InstTan2D<T>* d_inst = nullptr;
+  ChipInst<T>* d_chip = nullptr;  // the on-chip integrator's descriptors
   size_t smem = 0;
   int grid_cap = 148;
 
@@ -153,6 +155,7 @@ struct IntPlan {
     tan2d_tables<T>(n, h.data());
     PSG_CUDA_TRY(cudaMemcpy(tw, h.data(), sizeof(cpx<T>) * 2 * n, cudaMemcpyHostToDevice));
     PSG_CUDA_TRY(cudaMalloc(&d_inst, sizeof(InstTan2D<T>) * ng));
+    PSG_CUDA_TRY(cudaMalloc(&d_chip, sizeof(ChipInst<T>) * ng));
     smem = tan2d_smem<T>(n);
     const void* fns[3] = {tan2d_fn<T, 1>(n), tan2d_fn<T, 2>(n), tan2d_fn<T, 4>(n)};
     for (const void* f : fns)
@@ -170,6 +173,8 @@ struct IntPlan {
   void release() {
     if (d_inst) cudaFree(d_inst);
     d_inst = nullptr;
+    if (d_chip) cudaFree(d_chip);
+    d_chip = nullptr;
   }
 };
 
