@@ -32,10 +32,12 @@ FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", 
          "--ptxas-options=-O3", f"-I{INCLUDE}", f"-I{CSRC}"]
 
 # translation units of libpsgpu.so
-CORE = ["psg_api.cu", "psg_ns3d_api.cu", "psg_ns3d_f32.cu", "psg_ns3d_f64.cu",
+CORE = ["psg_api.cu", "psg_ns3d_api.cu",
         "psg_ns2d.cu", "psg_chip2d_f64.cu", "psg_chip2d_f32.cu",
         "psg_newton2d.cu", "psg_tan2d_f64.cu", "psg_tan2d_f32.cu",
         "psg_recurrence.cu", "psg_recurrence2d.cu"]
+# the 3D engine: one object per precision and grid size
+CORE3D = [(f"psg_ns3d_f{p}.cu", n) for n in (256, 128, 64, 32, 16) for p in (64, 32)]
 # host-side C of libpsgpu.so (parameter files, random starts, record I/O)
 HOST_SRC = ["psg_host.c"]
 # driver programs: name -> source (linked to libpsgpu.so)
@@ -98,6 +100,9 @@ def build(verbose: bool = False) -> str:
     core = [s for s in CORE if os.path.exists(os.path.join(CSRC, s))]
     dropins = {k: v for k, v in DROPINS.items() if os.path.exists(os.path.join(CSRC, v[0]))}
     with cf.ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as ex:
+        for s, n in CORE3D:
+            obj = os.path.join(OBJ, s.replace(".cu", f"_{n}.o"))
+            jobs.append(ex.submit(_compile, s, obj, (f"PSG_GRID={n}",)))
         for s in core:
             jobs.append(ex.submit(_compile, s, os.path.join(OBJ, s.replace(".cu", ".o"))))
         for name, (s, macro) in dropins.items():
@@ -107,6 +112,7 @@ def build(verbose: bool = False) -> str:
         for j in jobs:
             j.result()
     core_objs = [os.path.join(OBJ, s.replace(".cu", ".o")) for s in core]
+    core_objs += [os.path.join(OBJ, s.replace(".cu", f"_{n}.o")) for s, n in CORE3D]
     core_objs += [os.path.join(OBJ, s.replace(".c", ".o")) for s in HOST_SRC]
     libcore = os.path.join(LIB, "libpsgpu.so")
     if _stale(libcore, core_objs):

@@ -101,7 +101,16 @@ struct Engine3DBase {
   virtual int profile_read(double* ms, long* counts) = 0;
 };
 
-Engine3DBase* make_engine3d_f32();
-Engine3DBase* make_engine3d_f64();
+// the engine of precision T at an N^3 grid, N = 16 .. 256
+template <typename T, int N>
+Engine3DBase* make_engine3d();
+#define PSG_ENGINE3D_DECLARE(T)                                                        \
+  template <> Engine3DBase* make_engine3d<T, 16>();                                   \
+  template <> Engine3DBase* make_engine3d<T, 32>();                                   \
+  template <> Engine3DBase* make_engine3d<T, 64>();                                   \
+  template <> Engine3DBase* make_engine3d<T, 128>();                                  \
+  template <> Engine3DBase* make_engine3d<T, 256>();
+PSG_ENGINE3D_DECLARE(float)
+PSG_ENGINE3D_DECLARE(double)
 
 }  // namespace psg

@@ -16,6 +16,18 @@ struct psg_ns3d {
     }                                                       \
   } while (0)
 
+template <typename T>
+static Engine3DBase* engine3d(int n) {
+  switch (n) {
+    case 16: return make_engine3d<T, 16>();
+    case 32: return make_engine3d<T, 32>();
+    case 64: return make_engine3d<T, 64>();
+    case 128: return make_engine3d<T, 128>();
+    case 256: return make_engine3d<T, 256>();
+  }
+  return nullptr;
+}
+
 extern "C" int psg_ns3d_create(psg_ns3d** out, int n, double alpha, int scheme, int precision) {
   if (!out) { psg_set_error("null output handle"); return PSG_ERR_ARG; }
   *out = nullptr;
@@ -26,7 +38,12 @@ extern "C" int psg_ns3d_create(psg_ns3d** out, int n, double alpha, int scheme, 
     return PSG_ERR_UNSUPPORTED;
   }
   psg_ns3d* h = new psg_ns3d();
-  h->e = (precision == 64) ? make_engine3d_f64() : make_engine3d_f32();
+  h->e = (precision == 64) ? engine3d<double>(n) : engine3d<float>(n);
+  if (!h->e) {
+    delete h;
+    psg_set_error("3D grid size %d unsupported (powers of two 16..256)", n);
+    return PSG_ERR_UNSUPPORTED;
+  }
   int rc = h->e->init(n, alpha, scheme);
   if (rc) { delete h->e; delete h; return rc; }
   *out = h;

@@ -1,3 +1,5 @@
-// psg_ns3d_f64.cu -- FP64 instantiation of the 3D engine (kernels for every grid size).
+// psg_ns3d_f64.cu -- FP64 3D engine of one grid size, PSG_GRID (compiled once per size, so that
+// the sizes build in parallel).
 #include "psg_ns3d_impl.cuh"
-psg::Engine3DBase* psg::make_engine3d_f64() { return new psg::Engine3D<double>(); }
+template <>
+psg::Engine3DBase* psg::make_engine3d<double, PSG_GRID>() { return new psg::Engine3D<double, PSG_GRID>(); }

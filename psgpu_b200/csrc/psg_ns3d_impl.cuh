@@ -60,6 +60,38 @@ __device__ __forceinline__ bool keep_mode(int ix, int ky, int kz, int K, T alpha
   return !(wk > lim * lim);
 }
 
+// The kept modes lie in the ball |k| <= K - 1/2.  ball_reach: the largest m with
+// s + m^2 inside it (s the squares of the other wavenumbers), -1 if s is outside.
+// K^2 - K - s is an integer and (K - 1/2)^2 - s lies 1/4 above it, so the FP32
+// root never rounds across an integer.
+template <int N>
+__device__ __forceinline__ int ball_reach(int s) {
+  const int q = Box<N>::K * Box<N>::K - Box<N>::K - s;
+  return q < 0 ? -1 : (int)sqrtf((float)q + 0.25f);
+}
+// Reach in kz of the tile (xt, ky) and in ky of the tile column xt, taken at the
+// tile's lowest kx.  Outside them every mode of the stage state is zero, and
+// every mode the passes produce is masked away: pass A transforms no such tile
+// and loads no such rows, pass B reads no such rows, pass D stores none, pass E
+// updates none of them (256^3: 17% of the tiles of A and E, 45% of the state's
+// modes).  `full` (a device flag, null or PSG_WHOLE_BOX) lifts this: a state that
+// still holds truncated modes, as an uploaded one may, takes part with all of
+// its box.
+#define PSG_WHOLE_BOX reinterpret_cast<const int*>(1)
+__device__ __forceinline__ bool whole_box(const int* full) {
+  return full && (full == PSG_WHOLE_BOX || *full);
+}
+template <int N>
+__device__ __forceinline__ int tile_reach_z(bool all, int xt, int iky) {
+  const int kx = xt * kTileW, ky = iky - Box<N>::K;
+  return all ? Box<N>::K : ball_reach<N>(kx * kx + ky * ky);
+}
+template <int N>
+__device__ __forceinline__ int tile_reach_y(bool all, int xt) {
+  const int kx = xt * kTileW, r = ball_reach<N>(kx * kx);
+  return all ? Box<N>::K : r > 0 ? r : 0;
+}
+
 template <typename T>
 __device__ __forceinline__ T wkinv(T wk) {
   return (T)1 / (wk > (T)0.001 ? wk : (T)0.001);
@@ -147,25 +179,25 @@ __device__ __forceinline__ cpx<T> spec_op(int op, int comp, const cpx<T>* x, T k
 template <typename T, int N, int NC, typename Src>
 __device__ __forceinline__ bool a_stage(const Geom3<T>& g, Src src_comp, const cpx<T>* __restrict__ tw,
                                         cpx<T>* s_in, cpx<T>* s_tw, T* s_wk, uint64_t* s_bar,
-                                        int* s_ok, int* status) {
+                                        int* s_ok, int* status, int zm) {
   constexpr int W = kTileW;
   constexpr int Y = Box<N>::Y, K = Box<N>::K;
   const int tid = threadIdx.x, nth = blockDim.x;
   const int xt = blockIdx.x, iky = blockIdx.y;
   const long tile = ((long)xt * Y + iky) * Y * W;
-  pdl_trigger();
+  const int r0 = (K - zm) * W, rn = (2 * zm + 1) * W;  // the rows within the tile's reach
   if (tid == 0) mbar_init(s_bar, 1);
   __syncthreads();
   pdl_wait();
   if (tid == 0) {
-    mbar_expect_tx(s_bar, (uint32_t)(NC * Y * W * sizeof(cpx<T>)));
+    mbar_expect_tx(s_bar, (uint32_t)(NC * rn * sizeof(cpx<T>)));
     for (int q = 0; q < NC; ++q)
-      bulk_g2s(s_in + q * Y * W, src_comp(q) + tile, (uint32_t)(Y * W * sizeof(cpx<T>)), s_bar);
+      bulk_g2s(s_in + q * Y * W + r0, src_comp(q) + tile + r0, (uint32_t)(rn * sizeof(cpx<T>)), s_bar);
   }
   // the tables while the copy is in flight
   for (int i = tid; i < N; i += nth) s_tw[i] = tw[i];
   const bool mirror = (xt == 0) && (iky <= K);
-  for (int idx = tid; idx < Y * W; idx += nth) {
+  for (int idx = r0 + tid; idx < r0 + rn; idx += nth) {
     const int ikz = idx / W, cc = idx % W, ikx = xt * W + cc;
     bool ll;
     if (ikx >= Box<N>::X) ll = false;
@@ -179,8 +211,9 @@ __device__ __forceinline__ bool a_stage(const Geom3<T>& g, Src src_comp, const c
   if (!tile_wait(s_bar, s_ok, status)) return false;
   if (mirror) {
     const long mt = (long)(2 * K - iky) * Y * W;
-    for (int i = tid; i < NC * Y; i += nth) {
-      const int q = i / Y, ikz = i % Y;
+    const int nz = 2 * zm + 1;
+    for (int i = tid; i < NC * nz; i += nth) {
+      const int q = i / nz, ikz = K - zm + i % nz;
       cpx<T>* d = s_in + q * Y * W + ikz * W;
       if (iky == K && ikz == K) *d = czero<T>();
       else if (!(iky == K && ikz > K)) *d = cconj(src_comp(q)[mt + (long)(2 * K - ikz) * W]);
@@ -194,7 +227,7 @@ template <typename T, int N, int NC, int NF, int MODE = 0, int NG = 2>
 __global__ void __launch_bounds__(NG * kTileW * LineFFT<N, 1, T>::G,
                                   sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : (NG == 2 ? 3 : 2))
 pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __restrict__ tw,
-       int mask_vel, int* status, Fields4<T> in2 = Fields4<T>{}, int ops = 0) {
+       int mask_vel, int* status, const int* __restrict__ full, Fields4<T> in2 = Fields4<T>{}, int ops = 0) {
   using F = LineFFT<N, +1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
@@ -218,7 +251,10 @@ pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __rest
     if (MODE == 2 && q == 4) return in2.c[0];
     return in.c[q];
   };
-  if (!a_stage<T, N, NC>(g, src_comp, tw, s_in, s_tw, s_wk, &s_bar, &s_ok, status)) return;
+  pdl_trigger();
+  const int zm = tile_reach_z<N>(whole_box(full), xt, iky);
+  if (zm < 0) return;
+  if (!a_stage<T, N, NC>(g, src_comp, tw, s_in, s_tw, s_wk, &s_bar, &s_ok, status, zm)) return;
 
   const int ikx = xt * W + c;
   const T kx = (T)ikx * g.alpha;
@@ -234,7 +270,7 @@ pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __rest
       const int ikz = row_to_box(F::in_index(gi, e), K, N);
       const int o = ikz * W + c;
       cpx<T> r = czero<T>();
-      if (ikz >= 0 && live) {
+      if (ikz >= K - zm && ikz <= K + zm && live) {
         const T kz = (T)(ikz - K);
         const T tk = s_wk[o];
         if (MODE == 1) {
@@ -295,7 +331,7 @@ pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __rest
 template <int N, int NC, int NF>
 __global__ void __launch_bounds__(kTileW * LineFFT<N, 1, float>::G, 3)
 pass_a_pk(Geom3<float> g, Fields4<float> in, cpx<float>* __restrict__ out,
-          const cpx<float>* __restrict__ tw, int mask_vel, int* status) {
+          const cpx<float>* __restrict__ tw, int mask_vel, int* status, const int* __restrict__ full) {
   using T = float;
   using F = LineFFT<N, +1, T>;
   using F2 = LineFFT2<N, +1>;
@@ -312,7 +348,10 @@ pass_a_pk(Geom3<float> g, Fields4<float> in, cpx<float>* __restrict__ out,
   const int tid = threadIdx.x, c = tid % W, gi = tid / W;
   const int xt = blockIdx.x, iky = blockIdx.y;
   auto src_comp = [&](int q) -> const cpx<T>* { return in.c[q]; };
-  if (!a_stage<T, N, NC>(g, src_comp, tw, s_in, s_tw, s_wk, &s_bar, &s_ok, status)) return;
+  pdl_trigger();
+  const int zm = tile_reach_z<N>(whole_box(full), xt, iky);
+  if (zm < 0) return;
+  if (!a_stage<T, N, NC>(g, src_comp, tw, s_in, s_tw, s_wk, &s_bar, &s_ok, status, zm)) return;
   const int ikx = xt * W + c;
   const T kx = (T)ikx * g.alpha, ky = (T)(iky - K);
   const bool live = ikx < Box<N>::X;
@@ -342,7 +381,7 @@ pass_a_pk(Geom3<float> g, Fields4<float> in, cpx<float>* __restrict__ out,
       const int ikz = row_to_box(F::in_index(gi, e), K, N);
       const int o = ikz * W + c;
       cpx<T> a = czero<T>(), b = czero<T>();
-      if (ikz >= 0 && live) {
+      if (ikz >= K - zm && ikz <= K + zm && live) {
         const T kz = (T)(ikz - K), tk = s_wk[o];
         a = value(f0, o, kz, tk);
         if (two) b = value(f0 + 1, o, kz, tk);
@@ -369,7 +408,7 @@ pass_a_pk(Geom3<float> g, Fields4<float> in, cpx<float>* __restrict__ out,
 template <typename T, int N>
 __global__ void __launch_bounds__(kTileW * LineFFT<N, 1, T>::G)
 pass_b(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
-       const cpx<T>* __restrict__ tw, int* status) {
+       const cpx<T>* __restrict__ tw, int* status, const int* __restrict__ full) {
   using F = LineFFT<N, +1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
@@ -385,12 +424,14 @@ pass_b(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
   const int xt = blockIdx.x, z = blockIdx.y, f = blockIdx.z;
   pdl_trigger();
   if (tid == 0) mbar_init(&s_bar, 1);
+  const int ym = tile_reach_y<N>(whole_box(full), xt);
   __syncthreads();
   pdl_wait();
   if (tid == 0) {
-    mbar_expect_tx(&s_bar, (uint32_t)(Y * W * sizeof(cpx<T>)));
-    bulk_g2s(s_in, in + (((long)f * XT + xt) * N + z) * Y * W, (uint32_t)(Y * W * sizeof(cpx<T>)),
-             &s_bar);
+    const int r0 = (K - ym) * W;
+    const uint32_t bytes = (uint32_t)((2 * ym + 1) * W * sizeof(cpx<T>));
+    mbar_expect_tx(&s_bar, bytes);
+    bulk_g2s(s_in + r0, in + (((long)f * XT + xt) * N + z) * Y * W + r0, bytes, &s_bar);
   }
   for (int i = tid; i < N; i += blockDim.x) s_tw[i] = tw[i];
   if (!tile_wait(&s_bar, &s_ok, status)) return;
@@ -398,7 +439,7 @@ pass_b(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
 #pragma unroll
   for (int e = 0; e < F::E; ++e) {
     const int iky = row_to_box(F::in_index(gi, e), K, N);
-    v[e] = iky >= 0 ? s_in[iky * W + c] : czero<T>();
+    v[e] = (iky >= K - ym && iky <= K + ym) ? s_in[iky * W + c] : czero<T>();
   }
   __syncthreads();
   F::run(v, gi, s_tw, s_in + c * SX, BlockSync());
@@ -812,7 +853,7 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
 template <typename T, int N>
 __global__ void __launch_bounds__(kTileW * LineFFT<N, 1, T>::G)
 pass_d(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
-       const cpx<T>* __restrict__ tw, int* status) {
+       const cpx<T>* __restrict__ tw, int* status, const int* __restrict__ full) {
   using F = LineFFT<N, -1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
@@ -828,6 +869,7 @@ pass_d(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
   const int xt = blockIdx.x, z = blockIdx.y, f = blockIdx.z;
   pdl_trigger();
   if (tid == 0) mbar_init(&s_bar, 1);
+  const int ym = tile_reach_y<N>(whole_box(full), xt);
   __syncthreads();
   pdl_wait();
   if (tid == 0) {
@@ -847,7 +889,7 @@ pass_d(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
 #pragma unroll
   for (int e = 0; e < F::E; ++e) {
     const int iky = row_to_box(F::out_index(gi, e), K, N);
-    if (iky >= 0) dst[(long)iky * N * W] = v[e];
+    if (iky >= K - ym && iky <= K + ym) dst[(long)iky * N * W] = v[e];
   }
 }
 
@@ -1091,7 +1133,7 @@ struct GroupSync {
 template <typename T, int N, int NO, int SCHEME>
 __global__ void __launch_bounds__(2 * kTileW * LineFFT<N, 1, T>::G, sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : 3)
 pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw, Regs<T> R,
-       StepParams<T> p, int stage, int* status) {
+       StepParams<T> p, int stage, int* status, const int* __restrict__ full) {
   using F = LineFFT<N, -1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
@@ -1114,6 +1156,9 @@ pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw,
   const int tid = threadIdx.x, nth = blockDim.x, c = tid % W;
   const int xt = blockIdx.x, iky = blockIdx.y;
   pdl_trigger();
+  const int zm = tile_reach_z<N>(whole_box(full), xt, iky);
+  if (zm < 0) return;
+  const int u0 = (K - zm) * W, u1 = (K + zm + 1) * W;  // the modes to update
   if (tid == 0) mbar_init(&s_bar, 1);
   __syncthreads();
   const long tile = ((long)xt * Y + iky) * Y * W;
@@ -1125,18 +1170,19 @@ pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw,
       bulk_g2s(s_in + f * N * W, in + (((long)f * XT + xt) * Y + iky) * N * W, bytes, &s_bar);
     // the state tiles the update will read: fetch them into L2 while the
     // transforms run
-    const uint32_t sb = (uint32_t)(Y * W * sizeof(cpx<T>));
+    const uint32_t sb = (uint32_t)((u1 - u0) * sizeof(cpx<T>));
+    const long t0 = tile + u0;
     const int nc = (NO > 3) ? 4 : 3;
     for (int q = 0; q < nc; ++q) {
-      if (R.S.c[q]) bulk_prefetch_l2(R.S.c[q] + tile, sb);
+      if (R.S.c[q]) bulk_prefetch_l2(R.S.c[q] + t0, sb);
       const bool heun = (SCHEME == SCHEME_NS_HEUN || SCHEME == SCHEME_EULER_HEUN);
-      if (heun && stage == STAGE_HEUN_CORR && R.K1.c[q]) bulk_prefetch_l2(R.K1.c[q] + tile, sb);
-      if (SCHEME == SCHEME_BOUS_RK4 && R.X0.c[q]) bulk_prefetch_l2(R.X0.c[q] + tile, sb);
-      if (R.SC.c[q] && (heun || stage == STAGE_RK4)) bulk_prefetch_l2(R.SC.c[q] + tile, sb);
+      if (heun && stage == STAGE_HEUN_CORR && R.K1.c[q]) bulk_prefetch_l2(R.K1.c[q] + t0, sb);
+      if (SCHEME == SCHEME_BOUS_RK4 && R.X0.c[q]) bulk_prefetch_l2(R.X0.c[q] + t0, sb);
+      if (R.SC.c[q] && (heun || stage == STAGE_RK4)) bulk_prefetch_l2(R.SC.c[q] + t0, sb);
       if (!heun && stage == STAGE_RK4) {
-        if (R.K1.c[q]) bulk_prefetch_l2(R.K1.c[q] + tile, sb);
-        if (R.K2.c[q]) bulk_prefetch_l2(R.K2.c[q] + tile, sb);
-        if (R.K3.c[q]) bulk_prefetch_l2(R.K3.c[q] + tile, sb);
+        if (R.K1.c[q]) bulk_prefetch_l2(R.K1.c[q] + t0, sb);
+        if (R.K2.c[q]) bulk_prefetch_l2(R.K2.c[q] + t0, sb);
+        if (R.K3.c[q]) bulk_prefetch_l2(R.K3.c[q] + t0, sb);
       }
     }
   }
@@ -1168,7 +1214,7 @@ pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw,
     }
   }
   __syncthreads();
-  for (int idx = tid; idx < Y * W; idx += nth) {
+  for (int idx = u0 + tid; idx < u1; idx += nth) {
     const int ikz = idx / W, cc = idx % W, ikx = xt * W + cc;
     if (ikx >= Box<N>::X) continue;
     const long ik = tile + idx;
@@ -1303,7 +1349,7 @@ static __global__ void bflux_final(const double* __restrict__ part, int nblk, do
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void box_from_ref(Geom3<T> g, const double2* __restrict__ src, cpx<T>* __restrict__ dst,
-                             cpx<T>* __restrict__ low = nullptr) {
+                             cpx<T>* __restrict__ low = nullptr, int* __restrict__ full = nullptr) {
   const int W = kTileW;
   const long total = (long)g.XP * g.Y * g.Y;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
@@ -1319,6 +1365,10 @@ __global__ void box_from_ref(Geom3<T> g, const double2* __restrict__ src, cpx<T>
       const double2 s = src[((long)ikz * g.Y + iky) * g.X + ikx];
       v = cpx<T>{(T)s.x, (T)s.y};
       lo = cpx<T>{(T)(s.x - (double)v.x), (T)(s.y - (double)v.y)};
+      // a truncated mode that is not zero (or not a number): the passes take the
+      // whole box until the step has masked it
+      if (full && !(s.x == 0.0 && s.y == 0.0) && !keep_mode<T>(ikx, iky - g.K, ikz - g.K, g.K, g.alpha))
+        *full = 1;
     }
     dst[i] = v;
     if (low) low[i] = lo;
@@ -1691,7 +1741,7 @@ __global__ void bous_adj_combine(Geom3<T> g, T ri, T sinth, T costh, Fields4<T> 
 // ---------------------------------------------------------------------------
 // host engine
 // ---------------------------------------------------------------------------
-template <typename T>
+template <typename T, int NN>
 struct Engine3D final : Engine3DBase {
   Geom3<T> g{};
   int scheme = 0;
@@ -1702,6 +1752,14 @@ struct Engine3D final : Engine3DBase {
   StepParams<T> prm{};
   cudaStream_t stream = 0;
   int first_rhs = 1;     // mask velocity on the first evaluation after an upload
+  // Truncated modes of the state: an upload that brings some sets its flag,
+  // d_full[slot].  Every upload takes the next of the zeroed flags, so that only
+  // one in kFullSlots clears them.  fresh: no step has masked the state since the upload;
+  // exposed: the caller holds the state's device pointers and may write any mode.
+  static constexpr int kFullSlots = 256;
+  int* d_full = nullptr;
+  int slot = 0;
+  bool fresh = true, exposed = false;
   cpx<T>* pool = nullptr;
   cpx<T>* tw = nullptr;
   T* dump = nullptr;     // physical fields of the last step (Heun schemes)
@@ -1807,47 +1865,19 @@ struct Engine3D final : Engine3DBase {
   }
   size_t smem_e() const { return smem_e_no(nfo); }
   int col_stride() const {
-    switch (g.n) {
-      case 16: return ColStride<LineFFT<16, 1, T>::SMEM>::value;
-      case 32: return ColStride<LineFFT<32, 1, T>::SMEM>::value;
-      case 64: return ColStride<LineFFT<64, 1, T>::SMEM>::value;
-      case 128: return ColStride<LineFFT<128, 1, T>::SMEM>::value;
-      default: return ColStride<LineFFT<256, 1, T>::SMEM>::value;
-    }
+    return ColStride<LineFFT<NN, 1, T>::SMEM>::value;
   }
   int row_stride() const {
-    switch (g.n) {
-      case 16: return RowOps<T, 16>::SX;
-      case 32: return RowOps<T, 32>::SX;
-      case 64: return RowOps<T, 64>::SX;
-      case 128: return RowOps<T, 128>::SX;
-      default: return RowOps<T, 256>::SX;
-    }
+    return RowOps<T, NN>::SX;
   }
   int fft_g() const {
-    switch (g.n) {
-      case 16: return LineFFT<16, 1, T>::G;
-      case 32: return LineFFT<32, 1, T>::G;
-      case 64: return LineFFT<64, 1, T>::G;
-      case 128: return LineFFT<128, 1, T>::G;
-      default: return LineFFT<256, 1, T>::G;
-    }
+    return LineFFT<NN, 1, T>::G;
   }
   int fft_smem() const {
-    switch (g.n) {
-      case 16: return LineFFT<16, 1, T>::SMEM;
-      case 32: return LineFFT<32, 1, T>::SMEM;
-      case 64: return LineFFT<64, 1, T>::SMEM;
-      case 128: return LineFFT<128, 1, T>::SMEM;
-      default: return LineFFT<256, 1, T>::SMEM;
-    }
+    return LineFFT<NN, 1, T>::SMEM;
   }
 
   int init(int n, double alpha, int scheme_) override {
-    if (!(n == 16 || n == 32 || n == 64 || n == 128 || n == 256)) {
-      psg_set_error("3D grid size %d unsupported (powers of two 16..256)", n);
-      return PSG_ERR_UNSUPPORTED;
-    }
     g.n = n; g.K = n / 3; g.X = g.K + 1; g.Y = 2 * g.K + 1;
     g.XP = (g.X + kTileW - 1) / kTileW * kTileW;
     g.alpha = (T)alpha;
@@ -1888,17 +1918,13 @@ struct Engine3D final : Engine3DBase {
     // twiddle tables: the plain plan (column passes, inverse x rows) and the
     // swapped plan (forward x rows)
     std::vector<cpx<T>> h(2 * n);
-    switch (n) {
-      case 16: LineFFT<16, 1, T>::host_table(h.data()); LineFFT<16, 1, T, true>::host_table(h.data() + n); break;
-      case 32: LineFFT<32, 1, T>::host_table(h.data()); LineFFT<32, 1, T, true>::host_table(h.data() + n); break;
-      case 64: LineFFT<64, 1, T>::host_table(h.data()); LineFFT<64, 1, T, true>::host_table(h.data() + n); break;
-      case 128: LineFFT<128, 1, T>::host_table(h.data()); LineFFT<128, 1, T, true>::host_table(h.data() + n); break;
-      default: LineFFT<256, 1, T>::host_table(h.data()); LineFFT<256, 1, T, true>::host_table(h.data() + n); break;
-    }
+    LineFFT<NN, 1, T>::host_table(h.data());
+    LineFFT<NN, 1, T, true>::host_table(h.data() + n);
     PSG_CUDA_TRY(cudaMemcpy(tw, h.data(), sizeof(cpx<T>) * 2 * n, cudaMemcpyHostToDevice));
     PSG_CUDA_TRY(cudaMalloc(&stage_h, sizeof(double2) * (long)g.Y * g.Y * g.X));
-    PSG_CUDA_TRY(cudaMalloc(&d_status, sizeof(int)));
-    PSG_CUDA_TRY(cudaMemset(d_status, 0, sizeof(int)));
+    PSG_CUDA_TRY(cudaMalloc(&d_status, sizeof(int) * (1 + kFullSlots)));
+    PSG_CUDA_TRY(cudaMemset(d_status, 0, sizeof(int) * (1 + kFullSlots)));
+    d_full = d_status + 1;
     if (scheme == SCHEME_NS_HEUN || scheme == SCHEME_EULER_HEUN)
       PSG_CUDA_TRY(cudaMalloc(&dump, sizeof(T) * 3L * n * n * n));
     if (int rc = set_smem_limits()) return rc;
@@ -2143,13 +2169,8 @@ struct Engine3D final : Engine3DBase {
   }
   int autotune() override {
     int rc;
-    switch (g.n) {
-      case 16: rc = autotune_n<16>(); return rc ? rc : autotune_a_n<16>();
-      case 32: rc = autotune_n<32>(); return rc ? rc : autotune_a_n<32>();
-      case 64: rc = autotune_n<64>(); return rc ? rc : autotune_a_n<64>();
-      case 128: rc = autotune_n<128>(); return rc ? rc : autotune_a_n<128>();
-      default: rc = autotune_n<256>(); return rc ? rc : autotune_a_n<256>();
-    }
+    rc = autotune_n<NN>();
+    return rc ? rc : autotune_a_n<NN>();
   }
   int tuning_a(int* packed, float* ms) override {
     if (packed) *packed = a_pk ? 1 : 0;
@@ -2163,13 +2184,7 @@ struct Engine3D final : Engine3DBase {
     return PSG_OK;
   }
   int set_smem_limits() {
-    switch (g.n) {
-      case 16: return set_smem_limits_n<16>();
-      case 32: return set_smem_limits_n<32>();
-      case 64: return set_smem_limits_n<64>();
-      case 128: return set_smem_limits_n<128>();
-      default: return set_smem_limits_n<256>();
-    }
+    return set_smem_limits_n<NN>();
   }
 
   int sync() override { return check_status(); }
@@ -2192,10 +2207,21 @@ struct Engine3D final : Engine3DBase {
     return R.X0;
   }
 
+  // The passes' `full` flag for a right-hand side of `stage`: null when every
+  // truncated mode of the state is known to be zero.  The Euler predictor keeps
+  // truncated modes, a derivative writes them, and a forced mode outside the
+  // ball enters the RK4 stages.
+  const int* full_flag(int stage) const {
+    const bool forced_out = (scheme == SCHEME_NS_RK4 || scheme == SCHEME_BOUS_RK4) &&
+                            prm.ampfor != (T)0 && !(prm.kf >= (T)1 && prm.kf <= (T)g.K - (T)0.5);
+    if (scheme == SCHEME_EULER_HEUN || stage == STAGE_DERIV || exposed || forced_out) return PSG_WHOLE_BOX;
+    return fresh ? d_full + slot : nullptr;
+  }
+
   // one right-hand-side evaluation followed by the stage update
   // pass A of the step's right-hand side, scalar or on packed transforms
   template <int N>
-  int launch_a(bool chain, bool packed, Fields4<T> in, int mv) {
+  int launch_a(bool chain, bool packed, Fields4<T> in, int mv, const int* full = nullptr) {
     constexpr int G = LineFFT<N, 1, T>::G;
     const int XT = g.XP / kTileW;
     const bool bous = (scheme == SCHEME_BOUS_RK4);
@@ -2203,17 +2229,17 @@ struct Engine3D final : Engine3DBase {
       if (packed && a_pk_ok) {
         if (bous)
           return launch_k(chain, pass_a_pk<N, 4, 9>, dim3(XT, g.Y), dim3(kTileW * G), smem_a_pk_n<N>(4),
-                          g, in, B1, tw, mv, d_status);
+                          g, in, B1, tw, mv, d_status, full);
         return launch_k(chain, pass_a_pk<N, 3, 6>, dim3(XT, g.Y), dim3(kTileW * G), smem_a_pk_n<N>(3), g,
-                        in, B1, tw, mv, d_status);
+                        in, B1, tw, mv, d_status, full);
       }
     }
     const Fields4<T> none{};
     if (bous)
       return launch_k(chain, pass_a<T, N, 4, 9, 0, 3>, dim3(XT, g.Y), dim3(3 * kTileW * G), smem_a(), g,
-                      in, B1, tw, mv, d_status, none, 0);
+                      in, B1, tw, mv, d_status, full, none, 0);
     return launch_k(chain, pass_a<T, N, 3, 6>, dim3(XT, g.Y), dim3(2 * kTileW * G), smem_a(), g, in, B1,
-                    tw, mv, d_status, none, 0);
+                    tw, mv, d_status, full, none, 0);
   }
 
   // chain: the stream's last operation is the pass E of the previous
@@ -2229,10 +2255,11 @@ struct Engine3D final : Engine3DBase {
     first_rhs = 0;
     mark(-1);
     const dim3 blk2(2 * kTileW * G);
-    int rc = launch_a<N>(chain, a_pk, in, mv);
+    const int* full = full_flag(stage);
+    int rc = launch_a<N>(chain, a_pk, in, mv, full);
     if (rc) return rc;
     mark(0);
-    if ((rc = launch_k(true, pass_b<T, N>, dim3(XT, N, nfi), blk, smem_b(), g, B1, B2, tw, d_status)))
+    if ((rc = launch_k(true, pass_b<T, N>, dim3(XT, N, nfi), blk, smem_b(), g, B1, B2, tw, d_status, full)))
       return rc;
     mark(1);
     const T scale = (T)1 / ((T)N * (T)N * (T)N);
@@ -2243,28 +2270,30 @@ struct Engine3D final : Engine3DBase {
                           !want_umax && pdl != 2)))
       return rc;
     mark(2);
-    if ((rc = launch_k(true, pass_d<T, N>, dim3(XT, N, nfo), blk, smem_d(), g, B1, B2, tw, d_status)))
+    if ((rc = launch_k(true, pass_d<T, N>, dim3(XT, N, nfo), blk, smem_d(), g, B1, B2, tw, d_status, full)))
       return rc;
     mark(3);
     const dim3 ge(XT, g.Y);
     switch (scheme) {
       case SCHEME_NS_HEUN:
         rc = launch_k(true, pass_e<T, N, 3, SCHEME_NS_HEUN>, ge, blk2, smem_e(), g, B2, tw, R, prm,
-                      stage, d_status);
+                      stage, d_status, full);
         break;
       case SCHEME_EULER_HEUN:
         rc = launch_k(true, pass_e<T, N, 3, SCHEME_EULER_HEUN>, ge, blk2, smem_e(), g, B2, tw, R, prm,
-                      stage, d_status);
+                      stage, d_status, full);
         break;
       case SCHEME_NS_RK4:
         rc = launch_k(true, pass_e<T, N, 3, SCHEME_NS_RK4>, ge, blk2, smem_e(), g, B2, tw, R, prm,
-                      stage, d_status);
+                      stage, d_status, full);
         break;
       default:
         rc = launch_k(true, pass_e<T, N, 4, SCHEME_BOUS_RK4>, ge, blk2, smem_e(), g, B2, tw, R, prm,
-                      stage, d_status);
+                      stage, d_status, full);
     }
     if (rc) return rc;
+    // the final stage and the Heun predictor leave a masked state
+    if (stage == STAGE_RK4 || (stage == STAGE_HEUN_PRED && scheme == SCHEME_NS_HEUN)) fresh = false;
     mark(4);
     launches += 5;
     PSG_CUDA_TRY(cudaGetLastError());
@@ -2272,13 +2301,7 @@ struct Engine3D final : Engine3DBase {
   }
 
   int rhs(int stage, bool want_dump = false, bool want_umax = false, bool chain = false) {
-    switch (g.n) {
-      case 16: return rhs_n<16>(stage, want_dump, want_umax, chain);
-      case 32: return rhs_n<32>(stage, want_dump, want_umax, chain);
-      case 64: return rhs_n<64>(stage, want_dump, want_umax, chain);
-      case 128: return rhs_n<128>(stage, want_dump, want_umax, chain);
-      default: return rhs_n<256>(stage, want_dump, want_umax, chain);
-    }
+    return rhs_n<NN>(stage, want_dump, want_umax, chain);
   }
 
   // one full time step of length dt; dump: keep the physical vorticity of the
@@ -2298,14 +2321,26 @@ struct Engine3D final : Engine3DBase {
     return rhs(STAGE_RK4, false, false, true);
   }
 
+  // before an upload: its conversion kernels set the flag again where they find
+  // truncated modes
+  int state_from_outside() {
+    fresh = true;
+    if (++slot == kFullSlots) {
+      slot = 0;
+      PSG_CUDA_TRY(cudaMemsetAsync(d_full, 0, sizeof(int) * kFullSlots, stream));
+    }
+    return PSG_OK;
+  }
+
   // host FP64 boxes (reference layout) -> device state; RK4 schemes also set
   // the stage state X0 = S as the reference's setVelocity does.
   int upload(const double* const* comps) override {
     const long nref = (long)g.Y * g.Y * g.X;
+    if (int rc = state_from_outside()) return rc;
     for (int q = 0; q < nc; ++q) {
       PSG_CUDA_TRY(cudaMemcpyAsync(stage_h, comps[q], sizeof(double2) * nref,
                                    cudaMemcpyHostToDevice, stream));
-      box_from_ref<T><<<592, 256, 0, stream>>>(g, stage_h, R.S.c[q], R.SC.c[q]);
+      box_from_ref<T><<<592, 256, 0, stream>>>(g, stage_h, R.S.c[q], R.SC.c[q], d_full + slot);
       ++launches;
     }
     if (R.X0.c[0]) {
@@ -2338,6 +2373,7 @@ struct Engine3D final : Engine3DBase {
         psg_set_error("kept-mode upload needs page-locked host memory");
         return PSG_ERR_UNSUPPORTED;
       }
+    if (int rc = state_from_outside()) return rc;
     for (int q = 0; q < nc; ++q) {
       box_from_ref_kept<T><<<592, 256, 0, stream>>>(g, (const double2*)dp[q], R.S.c[q], R.SC.c[q]);
       ++launches;
@@ -2371,8 +2407,9 @@ struct Engine3D final : Engine3DBase {
   // device FP64 boxes (reference layout) <-> state, ordered on the engine's
   // stream, no host synchronisation
   int upload_device(const void* const* comps) override {
+    if (int rc = state_from_outside()) return rc;
     for (int q = 0; q < nc; ++q) {
-      box_from_ref<T><<<592, 256, 0, stream>>>(g, (const double2*)comps[q], R.S.c[q], R.SC.c[q]);
+      box_from_ref<T><<<592, 256, 0, stream>>>(g, (const double2*)comps[q], R.S.c[q], R.SC.c[q], d_full + slot);
       ++launches;
     }
     if (R.X0.c[0]) {
@@ -2456,13 +2493,7 @@ struct Engine3D final : Engine3DBase {
       return PSG_ERR_UNSUPPORTED;
     }
     int rc;
-    switch (g.n) {
-      case 16: rc = lin_attrs<16>(); break;
-      case 32: rc = lin_attrs<32>(); break;
-      case 64: rc = lin_attrs<64>(); break;
-      case 128: rc = lin_attrs<128>(); break;
-      default: rc = lin_attrs<256>(); break;
-    }
+    rc = lin_attrs<NN>();
     if (rc) return rc;
     // state-shaped registers (nc components) and product outputs (3, or 4 + 2)
     constexpr int kState = 15;
@@ -2490,14 +2521,14 @@ struct Engine3D final : Engine3DBase {
     const dim3 blk(kTileW * FG::G), blk2(2 * kTileW * FG::G);
     const int XT = g.XP / kTileW;
     pass_a<T, N, 6, 6, 1><<<dim3(XT, g.Y), blk2, smem_pair(), stream>>>(
-        g, b, B1, tw, 0, d_status, a, op_b | (op_a << 4));
-    pass_b<T, N><<<dim3(XT, N, 6), blk, smem_b(), stream>>>(g, B1, B2, tw, d_status);
+        g, b, B1, tw, 0, d_status, nullptr, a, op_b | (op_a << 4));
+    pass_b<T, N><<<dim3(XT, N, 6), blk, smem_b(), stream>>>(g, B1, B2, tw, d_status, nullptr);
     launch_c<N>(c_variant, (T)1 / ((T)N * (T)N * (T)N), nullptr, 6);
-    pass_d<T, N><<<dim3(XT, N, 3), blk, smem_d(), stream>>>(g, B1, B2, tw, d_status);
+    pass_d<T, N><<<dim3(XT, N, 3), blk, smem_d(), stream>>>(g, B1, B2, tw, d_status, nullptr);
     Regs<T> Rr{};
     Rr.K1 = out;
     pass_e<T, N, 3, SCHEME_RAW><<<dim3(XT, g.Y), blk2, smem_e_no(3), stream>>>(g, B2, tw, Rr, prm, 0,
-                                                                          d_status);
+                                                                          d_status, nullptr);
     launches += 5;
     PSG_CUDA_TRY(cudaGetLastError());
     return PSG_OK;
@@ -2512,27 +2543,21 @@ struct Engine3D final : Engine3DBase {
     Fields4<T> psi{};
     psi.c[0] = x.c[3];
     pass_a<T, N, 5, 7, 2><<<dim3(XT, g.Y), blk2, smem_a_nc(5), stream>>>(g, z, B1, tw, 0, d_status,
-                                                                         psi, 0);
-    pass_b<T, N><<<dim3(XT, N, 7), blk, smem_b(), stream>>>(g, B1, B2, tw, d_status);
+                                                                         nullptr, psi, 0);
+    pass_b<T, N><<<dim3(XT, N, 7), blk, smem_b(), stream>>>(g, B1, B2, tw, d_status, nullptr);
     launch_c<N>(c_variant, (T)1 / ((T)N * (T)N * (T)N), nullptr, 7);
-    pass_d<T, N><<<dim3(XT, N, 6), blk, smem_d(), stream>>>(g, B1, B2, tw, d_status);
+    pass_d<T, N><<<dim3(XT, N, 6), blk, smem_d(), stream>>>(g, B1, B2, tw, d_status, nullptr);
     Regs<T> Rr{};
     Rr.K1 = SA;
     Rr.K2 = SB;
     pass_e<T, N, 6, SCHEME_RAW><<<dim3(XT, g.Y), blk2, smem_e_no(6), stream>>>(g, B2, tw, Rr, prm, 0,
-                                                                              d_status);
+                                                                              d_status, nullptr);
     launches += 5;
     PSG_CUDA_TRY(cudaGetLastError());
     return PSG_OK;
   }
   int scale_products(Fields4<T> z, Fields4<T> x) {
-    switch (g.n) {
-      case 16: return scale_products_n<16>(z, x);
-      case 32: return scale_products_n<32>(z, x);
-      case 64: return scale_products_n<64>(z, x);
-      case 128: return scale_products_n<128>(z, x);
-      default: return scale_products_n<256>(z, x);
-    }
+    return scale_products_n<NN>(z, x);
   }
 
   double norm2(Fields4<T> x) {
@@ -2550,13 +2575,7 @@ struct Engine3D final : Engine3DBase {
   }
 
   int bilinear(Fields4<T> b, int op_b, Fields4<T> a, int op_a, Fields4<T> out) {
-    switch (g.n) {
-      case 16: return bilinear_n<16>(b, op_b, a, op_a, out);
-      case 32: return bilinear_n<32>(b, op_b, a, op_a, out);
-      case 64: return bilinear_n<64>(b, op_b, a, op_a, out);
-      case 128: return bilinear_n<128>(b, op_b, a, op_a, out);
-      default: return bilinear_n<256>(b, op_b, a, op_a, out);
-    }
+    return bilinear_n<NN>(b, op_b, a, op_a, out);
   }
 
   // out = N'(z) x (tangent) or N'(z)^T x (adjoint)
@@ -2808,6 +2827,7 @@ struct Engine3D final : Engine3DBase {
   }
   int layout(int* xp, void** comps) override {
     if (xp) *xp = g.XP;
+    if (comps) exposed = true;
     if (comps)
       for (int q = 0; q < 4; ++q) comps[q] = (void*)R.S.c[q];
     return PSG_OK;
