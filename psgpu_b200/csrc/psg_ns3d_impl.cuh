@@ -1347,104 +1347,69 @@ static __global__ void bflux_final(const double* __restrict__ part, int nblk, do
 // ---------------------------------------------------------------------------
 // layout conversion between the reference's FP64 boxes and the tile layout
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void box_from_ref(Geom3<T> g, const double2* __restrict__ src, cpx<T>* __restrict__ dst,
-                             cpx<T>* __restrict__ low = nullptr, int* __restrict__ full = nullptr) {
-  const int W = kTileW;
-  const long total = (long)g.XP * g.Y * g.Y;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
-       i += (long)gridDim.x * blockDim.x) {
-    const int w = (int)(i % W);
-    long r = i / W;
-    const int ikz = (int)(r % g.Y); r /= g.Y;
-    const int iky = (int)(r % g.Y);
-    const int xt = (int)(r / g.Y);
-    const int ikx = xt * W + w;
+// One launch converts every component (blockIdx.y counts from q0): upload writes
+// the state, its carried error (FP32) and, for the RK4 schemes, the stage state,
+// in one pass over the boxes (one launch each and a copy from the state to the
+// stage state cost seven launches of a 32^3 upload and download, a seventh of a
+// one-step call).  `kept`: host boxes in page-locked memory that the kernels
+// address directly, on the kept modes only: the upload reads those (and stores
+// zero for every other mode of the state), the download leaves the other entries
+// of the host box alone.
+struct RefBoxes {
+  double2* p[4];
+};
+
+template <typename T, int N>
+__global__ void __launch_bounds__(256)
+box_from_ref(RefBoxes src, Fields4<T> dst, Fields4<T> low, Fields4<T> dst2, int q0, bool kept,
+             int* __restrict__ full) {
+  constexpr int W = kTileW, K = Box<N>::K, X = Box<N>::X, Y = Box<N>::Y;
+  constexpr int total = Box<N>::XP * Y * Y;
+  const int q = q0 + blockIdx.y;
+  const double2* __restrict__ s = src.p[q];
+  cpx<T>*d = dst.c[q], *lw = low.c[q], *d2 = dst2.c[q];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int w = i % W, r = i / W;
+    const int ikz = r % Y, iky = r / Y % Y, ikx = r / (Y * Y) * W + w;
     cpx<T> v = czero<T>(), lo = czero<T>();
-    if (ikx < g.X) {
-      const double2 s = src[((long)ikz * g.Y + iky) * g.X + ikx];
-      v = cpx<T>{(T)s.x, (T)s.y};
-      lo = cpx<T>{(T)(s.x - (double)v.x), (T)(s.y - (double)v.y)};
-      // a truncated mode that is not zero (or not a number): the passes take the
-      // whole box until the step has masked it
-      if (full && !(s.x == 0.0 && s.y == 0.0) && !keep_mode<T>(ikx, iky - g.K, ikz - g.K, g.K, g.alpha))
-        *full = 1;
+    if (ikx < X) {
+      const bool keep = keep_mode<T>(ikx, iky - K, ikz - K, K, (T)1);
+      if (keep || !kept) {
+        const double2 a = s[(ikz * Y + iky) * X + ikx];
+        v = cpx<T>{(T)a.x, (T)a.y};
+        lo = cpx<T>{(T)(a.x - (double)v.x), (T)(a.y - (double)v.y)};
+        // a truncated mode that is not zero (or not a number): the passes take
+        // the whole box until the step has masked it
+        if (full && !keep && !(a.x == 0.0 && a.y == 0.0)) *full = 1;
+      }
     }
-    dst[i] = v;
-    if (low) low[i] = lo;
+    d[i] = v;
+    if (lw) lw[i] = lo;
+    if (d2) d2[i] = v;
   }
 }
 
-template <typename T>
-__global__ void box_to_ref(Geom3<T> g, const cpx<T>* __restrict__ src, double2* __restrict__ dst,
-                           const cpx<T>* __restrict__ low = nullptr) {
-  const int W = kTileW;
-  const long total = (long)g.Y * g.Y * g.X;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
-       i += (long)gridDim.x * blockDim.x) {
-    const int ikx = (int)(i % g.X);
-    const long r = i / g.X;
-    const int iky = (int)(r % g.Y), ikz = (int)(r / g.Y);
-    const long j = (((long)(ikx / W) * g.Y + iky) * g.Y + ikz) * W + (ikx % W);
-    const cpx<T> s = src[j];
-    double2 v = make_double2((double)s.x, (double)s.y);
-    if (low) {
-      const cpx<T> c = low[j];
+template <typename T, int N>
+__global__ void __launch_bounds__(256)
+box_to_ref(Fields4<T> src, Fields4<T> low, RefBoxes dst, int q0, bool kept) {
+  constexpr int W = kTileW, K = Box<N>::K, X = Box<N>::X, Y = Box<N>::Y;
+  constexpr int total = X * Y * Y;
+  const int q = q0 + blockIdx.y;
+  const cpx<T>*s = src.c[q], *lw = low.c[q];
+  double2* __restrict__ d = dst.p[q];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int ikx = i % X, r = i / X;
+    const int iky = r % Y, ikz = r / Y;
+    if (kept && !keep_mode<T>(ikx, iky - K, ikz - K, K, (T)1)) continue;
+    const int j = ((ikx / W * Y + iky) * Y + ikz) * W + ikx % W;
+    const cpx<T> a = s[j];
+    double2 v = make_double2((double)a.x, (double)a.y);
+    if (lw) {
+      const cpx<T> c = lw[j];
       v.x += (double)c.x;
       v.y += (double)c.y;
     }
-    dst[i] = v;
-  }
-}
-
-// The same two conversions on the kept modes only, for host boxes in
-// page-locked memory that the kernels address directly: the upload reads the
-// kept modes (and stores zero for every other mode of the state), the download
-// writes the kept modes and leaves the other entries of the host box alone.
-template <typename T>
-__global__ void box_from_ref_kept(Geom3<T> g, const double2* __restrict__ src,
-                                  cpx<T>* __restrict__ dst, cpx<T>* __restrict__ low) {
-  const int W = kTileW;
-  const long total = (long)g.XP * g.Y * g.Y;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
-       i += (long)gridDim.x * blockDim.x) {
-    const int w = (int)(i % W);
-    long r = i / W;
-    const int ikz = (int)(r % g.Y); r /= g.Y;
-    const int iky = (int)(r % g.Y);
-    const int xt = (int)(r / g.Y);
-    const int ikx = xt * W + w;
-    cpx<T> v = czero<T>(), lo = czero<T>();
-    if (ikx < g.X && keep_mode<T>(ikx, iky - g.K, ikz - g.K, g.K, g.alpha)) {
-      const double2 s = src[((long)ikz * g.Y + iky) * g.X + ikx];
-      v = cpx<T>{(T)s.x, (T)s.y};
-      lo = cpx<T>{(T)(s.x - (double)v.x), (T)(s.y - (double)v.y)};
-    }
-    dst[i] = v;
-    if (low) low[i] = lo;
-  }
-}
-
-template <typename T>
-__global__ void box_to_ref_kept(Geom3<T> g, const cpx<T>* __restrict__ src, double2* __restrict__ dst,
-                                const cpx<T>* __restrict__ low) {
-  const int W = kTileW;
-  const long total = (long)g.Y * g.Y * g.X;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
-       i += (long)gridDim.x * blockDim.x) {
-    const int ikx = (int)(i % g.X);
-    const long r = i / g.X;
-    const int iky = (int)(r % g.Y), ikz = (int)(r / g.Y);
-    if (!keep_mode<T>(ikx, iky - g.K, ikz - g.K, g.K, g.alpha)) continue;
-    const long j = (((long)(ikx / W) * g.Y + iky) * g.Y + ikz) * W + (ikx % W);
-    const cpx<T> s = src[j];
-    double2 v = make_double2((double)s.x, (double)s.y);
-    if (low) {
-      const cpx<T> c = low[j];
-      v.x += (double)c.x;
-      v.y += (double)c.y;
-    }
-    dst[i] = v;
+    d[i] = v;
   }
 }
 
@@ -2321,6 +2286,28 @@ struct Engine3D final : Engine3DBase {
     return rhs(STAGE_RK4, false, false, true);
   }
 
+  // boxes in the reference layout <-> fields of the engine, components q0 .. q0 + m - 1
+  int from_ref(const void* const* comps, int q0, int m, Fields4<T> dst, Fields4<T> low, Fields4<T> dst2,
+               bool kept, int* full) {
+    RefBoxes b{};
+    for (int q = 0; q < m; ++q) b.p[q0 + q] = (double2*)comps[q];
+    const int total = Box<NN>::XP * Box<NN>::Y * Box<NN>::Y;
+    box_from_ref<T, NN><<<dim3(std::min((total + 255) / 256, 1184), m), 256, 0, stream>>>(b, dst, low, dst2, q0,
+                                                                                       kept, full);
+    ++launches;
+    PSG_CUDA_TRY(cudaGetLastError());
+    return PSG_OK;
+  }
+  int to_ref(Fields4<T> src, Fields4<T> low, void* const* comps, int q0, int m, bool kept) {
+    RefBoxes b{};
+    for (int q = 0; q < m; ++q) b.p[q0 + q] = (double2*)comps[q];
+    const int total = Box<NN>::X * Box<NN>::Y * Box<NN>::Y;
+    box_to_ref<T, NN><<<dim3(std::min((total + 255) / 256, 1184), m), 256, 0, stream>>>(src, low, b, q0, kept);
+    ++launches;
+    PSG_CUDA_TRY(cudaGetLastError());
+    return PSG_OK;
+  }
+
   // before an upload: its conversion kernels set the flag again where they find
   // truncated modes
   int state_from_outside() {
@@ -2340,16 +2327,14 @@ struct Engine3D final : Engine3DBase {
     for (int q = 0; q < nc; ++q) {
       PSG_CUDA_TRY(cudaMemcpyAsync(stage_h, comps[q], sizeof(double2) * nref,
                                    cudaMemcpyHostToDevice, stream));
-      box_from_ref<T><<<592, 256, 0, stream>>>(g, stage_h, R.S.c[q], R.SC.c[q], d_full + slot);
-      ++launches;
+      const void* src = stage_h;
+      if (int rc = from_ref(&src, q, 1, R.S, R.SC, R.X0, false, d_full + slot)) return rc;
     }
-    if (R.X0.c[0]) {
-      copy_fields<T><<<592, 256, 0, stream>>>(R.S, R.X0, nc, box);
-      ++launches;
-    }
+    return uploaded();
+  }
+  int uploaded() {
     first_rhs = 1;
     lin_dx = false;
-    PSG_CUDA_TRY(cudaGetLastError());
     return PSG_OK;
   }
 
@@ -2374,18 +2359,8 @@ struct Engine3D final : Engine3DBase {
         return PSG_ERR_UNSUPPORTED;
       }
     if (int rc = state_from_outside()) return rc;
-    for (int q = 0; q < nc; ++q) {
-      box_from_ref_kept<T><<<592, 256, 0, stream>>>(g, (const double2*)dp[q], R.S.c[q], R.SC.c[q]);
-      ++launches;
-    }
-    if (R.X0.c[0]) {
-      copy_fields<T><<<592, 256, 0, stream>>>(R.S, R.X0, nc, box);
-      ++launches;
-    }
-    first_rhs = 1;
-    lin_dx = false;
-    PSG_CUDA_TRY(cudaGetLastError());
-    return PSG_OK;
+    if (int rc = from_ref(dp, 0, nc, R.S, R.SC, R.X0, true, nullptr)) return rc;
+    return uploaded();
   }
   int download_kept(double* const* comps) override {
     void* dp[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -2395,11 +2370,7 @@ struct Engine3D final : Engine3DBase {
         return PSG_ERR_UNSUPPORTED;
       }
     if (int rc = check_status()) return rc;
-    for (int q = 0; q < nc; ++q) {
-      box_to_ref_kept<T><<<592, 256, 0, stream>>>(g, R.S.c[q], (double2*)dp[q], R.SC.c[q]);
-      ++launches;
-    }
-    PSG_CUDA_TRY(cudaGetLastError());
+    if (int rc = to_ref(R.S, R.SC, dp, 0, nc, true)) return rc;
     PSG_CUDA_TRY(cudaStreamSynchronize(stream));
     return PSG_OK;
   }
@@ -2408,27 +2379,10 @@ struct Engine3D final : Engine3DBase {
   // stream, no host synchronisation
   int upload_device(const void* const* comps) override {
     if (int rc = state_from_outside()) return rc;
-    for (int q = 0; q < nc; ++q) {
-      box_from_ref<T><<<592, 256, 0, stream>>>(g, (const double2*)comps[q], R.S.c[q], R.SC.c[q], d_full + slot);
-      ++launches;
-    }
-    if (R.X0.c[0]) {
-      copy_fields<T><<<592, 256, 0, stream>>>(R.S, R.X0, nc, box);
-      ++launches;
-    }
-    first_rhs = 1;
-    lin_dx = false;
-    PSG_CUDA_TRY(cudaGetLastError());
-    return PSG_OK;
+    if (int rc = from_ref(comps, 0, nc, R.S, R.SC, R.X0, false, d_full + slot)) return rc;
+    return uploaded();
   }
-  int download_device(void* const* comps) override {
-    for (int q = 0; q < nc; ++q) {
-      box_to_ref<T><<<592, 256, 0, stream>>>(g, R.S.c[q], (double2*)comps[q], R.SC.c[q]);
-      ++launches;
-    }
-    PSG_CUDA_TRY(cudaGetLastError());
-    return PSG_OK;
-  }
+  int download_device(void* const* comps) override { return to_ref(R.S, R.SC, comps, 0, nc, false); }
 
   // ---------------------------------------------------------------- linearised step
   // pass A: staged tile [ncin][Y][W], twiddles, ng exchange groups, 1/k^2 table
@@ -2710,9 +2664,8 @@ struct Engine3D final : Engine3DBase {
   int linear(int mode, double dt, const void* const* in, void* const* out) override {
     int rc;
     if ((rc = lin_init())) return rc;
-    for (int q = 0; q < nc; ++q)
-      box_from_ref<T><<<592, 256, 0, stream>>>(g, (const double2*)in[q], LD.c[q], nullptr);
-    launches += nc;
+    const Fields4<T> none{};
+    if ((rc = from_ref(in, 0, nc, LD, none, none, false, nullptr))) return rc;
     Fields4<T> res = LD;
     switch (mode) {
       case 0:
@@ -2728,11 +2681,7 @@ struct Engine3D final : Engine3DBase {
       default: psg_set_error("linear mode %d unknown", mode); return PSG_ERR_ARG;
     }
     if (rc) return rc;
-    for (int q = 0; q < nc; ++q)
-      box_to_ref<T><<<592, 256, 0, stream>>>(g, res.c[q], (double2*)out[q], nullptr);
-    launches += nc;
-    PSG_CUDA_TRY(cudaGetLastError());
-    return PSG_OK;
+    return to_ref(res, none, out, 0, nc, false);
   }
 
   int set_forcing_form(int form) override {
@@ -2889,8 +2838,8 @@ struct Engine3D final : Engine3DBase {
     const long nref = (long)g.Y * g.Y * g.X;
     const Fields4<T>& F = src ? *src : R.S;
     for (int q = 0; q < nc; ++q) {
-      box_to_ref<T><<<592, 256, 0, stream>>>(g, F.c[q], stage_h, src ? nullptr : R.SC.c[q]);
-      ++launches;
+      void* dst = stage_h;
+      if (int rc = to_ref(F, src ? Fields4<T>{} : R.SC, &dst, q, 1, false)) return rc;
       PSG_CUDA_TRY(cudaMemcpyAsync(comps[q], stage_h, sizeof(double2) * nref,
                                    cudaMemcpyDeviceToHost, stream));
     }
