@@ -29,6 +29,7 @@ enum Scheme3D : int {
   SCHEME_NS_RK4 = 2,      // 3D_Boussinesq/src/kernels.h:331-621 without density
   SCHEME_BOUS_RK4 = 3,    // 3D_Boussinesq/src/kernels.h:331-621
   SCHEME_RAW = 4,         // pass E writes the masked transform itself (bilinear products)
+  SCHEME_LIN = 5,         // pass E forms the linearised step's right-hand sides
 };
 
 // stage codes of pass E

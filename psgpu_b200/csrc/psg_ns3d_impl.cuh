@@ -151,10 +151,10 @@ __device__ __forceinline__ bool tile_wait(uint64_t* bar, int* s_ok, int* status)
 // gradient) formed in registers; Hermitian completion of the kx = 0 plane.
 // grid (XT, Y): one [kz][W] tile of each state component.
 //
-// MODE 1 (pair): the two 3-vectors of a bilinear product, b = in (written to
-// the w slots 0-2 that pass C reads as w) and a = in2 (the u slots 3-5), each
-// passed through the spectral operator of `ops` (bits 0-3 for b, 4-7 for a:
-// OP_ID, OP_CURL = i k x, OP_BS = i k x / k^2) and masked to the kept modes.
+// MODE 3 / 4 (linearised step): the 3-vectors of the adjoint's and the tangent's
+// cross products, z = in and x = in2 passed through spectral operators (OP_ID,
+// OP_CURL = i k x, OP_BS = i k x / k^2) and masked to the kept modes: z, C x,
+// B z (adjoint, nine fields) and z, B z, x, B x (tangent, twelve).
 // MODE 2 (scale): the fields of the Boussinesq adjoint's scalar products,
 // [psi, i k rho, B w] from psi = in2.c[0] and (w, rho) = in.c[0..3].
 // ---------------------------------------------------------------------------
@@ -227,7 +227,7 @@ template <typename T, int N, int NC, int NF, int MODE = 0, int NG = 2>
 __global__ void __launch_bounds__(NG * kTileW * LineFFT<N, 1, T>::G,
                                   sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : (NG == 2 ? 3 : 2))
 pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __restrict__ tw,
-       int mask_vel, int* status, const int* __restrict__ full, Fields4<T> in2 = Fields4<T>{}, int ops = 0) {
+       int mask_vel, int* status, const int* __restrict__ full, Fields4<T> in2 = Fields4<T>{}) {
   using F = LineFFT<N, +1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
@@ -247,7 +247,7 @@ pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __rest
   const int c = ht % W, gi = ht / W;
   const int xt = blockIdx.x, iky = blockIdx.y;
   auto src_comp = [&](int q) -> const cpx<T>* {
-    if (MODE == 1 && q >= 3) return in2.c[q - 3];
+    if (MODE >= 3 && q >= 3) return in2.c[q - 3];
     if (MODE == 2 && q == 4) return in2.c[0];
     return in.c[q];
   };
@@ -273,12 +273,14 @@ pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __rest
       if (ikz >= K - zm && ikz <= K + zm && live) {
         const T kz = (T)(ikz - K);
         const T tk = s_wk[o];
-        if (MODE == 1) {
+        if (MODE >= 3) {
           if (tk > (T)0) {
-            const int sl = f / 3, comp = f % 3;
+            const int v3 = f / 3, comp = f % 3;  // which vector of the mode's list
+            const int sl = MODE == 3 ? (v3 == 1) : (v3 >= 2);
+            const int op = MODE == 3 ? (v3 == 0 ? OP_ID : v3 == 1 ? OP_CURL : OP_BS) : (v3 & 1) ? OP_BS : OP_ID;
             const cpx<T> x[3] = {s_in[(3 * sl) * Y * W + o], s_in[(3 * sl + 1) * Y * W + o],
                                  s_in[(3 * sl + 2) * Y * W + o]};
-            r = spec_op<T>((ops >> (4 * sl)) & 15, comp, x, kx, ky, kz, tk);
+            r = spec_op<T>(op, comp, x, kx, ky, kz, tk);
           }
         } else if (MODE == 2) {
           if (tk > (T)0) {
@@ -636,6 +638,11 @@ struct RowOps {
 // packed f32x2 transform (RowOps::c2r_quad / r2c_quad), with the exchange in
 // two halves through the scalar-sized buffer (1) or in one pass through a
 // buffer twice that size (2).
+// NF 9 + kLinAdj and 12 + kLinTan: the linearised step's fields (pass A, modes 3
+// and 4) and their cross products: adjoint -(z x Cx) and -(Cx x Bz), six fields
+// out, the transforms of C x shared by both; tangent -(Bx x z) - (Bz x x), summed
+// before the transform, three fields out.
+constexpr int kLinAdj = 100, kLinTan = 200;
 template <typename T, int N, int NF, int L, int ST, int PK = 0>
 __global__ void __launch_bounds__(L * LineFFT<N, 1, T>::G,
                                   (sizeof(T) == 4 && NF == 9 && L * LineFFT<N, 1, T>::G <= 128) ? 3 : 0)
@@ -648,10 +655,11 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
   constexpr int RPW = 32 / G, WPB = L / RPW;  // rows per warp tile, warps per block
   static_assert(L % RPW == 0, "whole warps per block");
   constexpr bool BOUS = (NF == 9);
+  constexpr int NI = NF % 100;  // fields read
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint64_t s_bar[WPB][2];
   constexpr int K = Box<N>::K, XP = Box<N>::XP, XT = Box<N>::XT;
-  constexpr int wtile_words = NF * RPW * XP;
+  constexpr int wtile_words = NI * RPW * XP;
   cpx<T>* s_buf = reinterpret_cast<cpx<T>*>(smem_raw);  // [WPB][ST][NF][RPW][XP]
   cpx<T>* s_tw = s_buf + WPB * ST * wtile_words;         // [2N]: plain | swapped plan
   cpx<T>* s_ex = s_tw + 2 * N;                           // [L][SX]
@@ -670,8 +678,8 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
   // the __syncwarp that precedes every call
   auto issue = [&](int t, int b) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(&bar[b], NF * bytes);
-    for (int f = 0; f < NF; ++f)
+    mbar_expect_tx(&bar[b], NI * bytes);
+    for (int f = 0; f < NI; ++f)
       bulk_g2s(s_w + b * wtile_words + f * RPW * XP, in + f * plane + (long)t * RPW * XP, bytes,
                &bar[b]);
   };
@@ -725,6 +733,51 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
 #pragma unroll
       for (int e = 0; e < E; ++e) p2[e] = ps[e] * ga[e] * hscale;
       R::r2c_pair(p1, p2, K, XP, gi, two, ex, dst + 4 * fstride, dst + 5 * fstride, tstride);
+      __syncwarp();
+      continue;
+    }
+    if constexpr (NF >= 100) {
+      // n -= a x b, scaled
+      auto cross = [&](const T (&a)[3][E], const T (&b)[3][E], T (&n)[3][E], T sc, bool add) {
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+            const T x = -(a[k1][e] * b[k2][e] - a[k2][e] * b[k1][e]) * sc;
+            n[k][e] = add ? n[k][e] + x : x;
+          }
+      };
+      T a[3][E], b3[3][E], n[3][E];
+      R::c2r_pair(src + 3 * fs, src + 4 * fs, K, gi, s_tw, ex, b3[0], b3[1]);
+      if constexpr (NF == 9 + kLinAdj) {
+        R::c2r_pair(src + 5 * fs, src, K, gi, s_tw, ex, b3[2], a[0]);
+        R::c2r_pair(src + fs, src + 2 * fs, K, gi, s_tw, ex, a[1], a[2]);
+        cross(a, b3, n, hscale, false);  // -(z x Cx)
+        R::r2c_pair(n[0], n[1], K, XP, gi, two, ex, dst, dst + fstride, tstride);
+        R::c2r_pair(src + 6 * fs, src + 7 * fs, K, gi, s_tw, ex, a[0], a[1]);
+        T last[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) last[e] = n[2][e];
+        R::c2r_pair(src + 8 * fs, nullptr, K, gi, s_tw, ex, a[2], n[2]);
+        release();
+        cross(b3, a, n, hscale, false);  // -(Cx x Bz)
+        R::r2c_pair(last, n[0], K, XP, gi, two, ex, dst + 2 * fstride, dst + 3 * fstride, tstride);
+        R::r2c_pair(n[1], n[2], K, XP, gi, two, ex, dst + 4 * fstride, dst + 5 * fstride, tstride);
+      } else {
+        R::c2r_pair(src + 5 * fs, src + 6 * fs, K, gi, s_tw, ex, b3[2], a[0]);
+        R::c2r_pair(src + 7 * fs, src + 8 * fs, K, gi, s_tw, ex, a[1], a[2]);
+        cross(b3, a, n, hscale, false);  // -(Bz x x)
+        R::c2r_pair(src + 9 * fs, src + 10 * fs, K, gi, s_tw, ex, a[0], a[1]);
+        R::c2r_pair(src + 11 * fs, src, K, gi, s_tw, ex, a[2], b3[0]);
+        R::c2r_pair(src + fs, src + 2 * fs, K, gi, s_tw, ex, b3[1], b3[2]);
+        release();
+        cross(a, b3, n, hscale, true);  // -(Bx x z)
+        R::r2c_pair(n[0], n[1], K, XP, gi, two, ex, dst, dst + fstride, tstride);
+#pragma unroll
+        for (int e = 0; e < E; ++e) n[2][e] *= (T)2;  // alone: no 1/2 of a split
+        R::r2c_pair(n[2], nullptr, K, XP, gi, two, ex, dst + 2 * fstride, nullptr, tstride);
+      }
       __syncwarp();
       continue;
     }
@@ -1172,7 +1225,7 @@ pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw,
     // transforms run
     const uint32_t sb = (uint32_t)((u1 - u0) * sizeof(cpx<T>));
     const long t0 = tile + u0;
-    const int nc = (NO > 3) ? 4 : 3;
+    const int nc = SCHEME == SCHEME_RAW || SCHEME == SCHEME_LIN ? 0 : (NO > 3) ? 4 : 3;
     for (int q = 0; q < nc; ++q) {
       if (R.S.c[q]) bulk_prefetch_l2(R.S.c[q] + t0, sb);
       const bool heun = (SCHEME == SCHEME_NS_HEUN || SCHEME == SCHEME_EULER_HEUN);
@@ -1224,6 +1277,23 @@ pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw,
     const cpx<T> V = s_in[(1 * N + R0 + ikz) * W + cc];
     const cpx<T> Wv = s_in[(2 * N + R0 + ikz) * W + cc];
     const cpx<T> RKv = (NO > 3) ? s_in[(3 * N + R0 + ikz) * W + cc] : czero<T>();
+    if (SCHEME == SCHEME_LIN) {
+      // right-hand sides of the linearised step into K1: tangent -C (sum of the
+      // products), adjoint -(B PA + PB)
+      const T LL = keep_mode<T>(ikx, iy, iz, Box<N>::K, g.alpha) ? (T)-1 : (T)0;
+      const T kz = (T)iz, wki = wkinv(kx * kx + ky * ky + kz * kz);
+      const cpx<T> a[3] = {U, V, Wv};
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        cpx<T> r = spec_op<T>(NO == 6 ? OP_BS : OP_CURL, q, a, kx, ky, kz, wki);
+        if (NO == 6) {
+          const cpx<T> b = s_in[((3 + q) * N + R0 + ikz) * W + cc];
+          r = cpx<T>{r.x + b.x, r.y + b.y};
+        }
+        R.K1.c[q][ik] = cpx<T>{LL * r.x, LL * r.y};
+      }
+      continue;
+    }
     if (SCHEME == SCHEME_RAW) {  // outputs 0-3 to K1, 4-5 to K2
       const T LL = keep_mode<T>(ikx, iy, iz, Box<N>::K, g.alpha) ? (T)1 : (T)0;
 #pragma unroll
@@ -1463,11 +1533,10 @@ template <typename T>
 __device__ __forceinline__ TileMode<T> tile_mode(const Geom3<T>& g, long i) {
   TileMode<T> m;
   const int W = kTileW;
-  const int w = (int)(i % W);
-  long q = i / W;
-  const int ikz = (int)(q % g.Y); q /= g.Y;
-  const int iky = (int)(q % g.Y);
-  const int ikx = (int)(q / g.Y) * W + w;
+  const unsigned j = (unsigned)i, yy = (unsigned)g.Y;  // a box is far below 2^32 modes
+  const int w = (int)(j % W);
+  const unsigned q = j / W;
+  const int ikz = (int)(q % yy), iky = (int)(q / yy % yy), ikx = (int)(q / yy / yy) * W + w;
   m.ok = ikx < g.X;
   m.keep = m.ok && keep_mode<T>(ikx, iky - g.K, ikz - g.K, g.K, g.alpha);
   m.kx = (T)ikx * g.alpha; m.ky = (T)(iky - g.K); m.kz = (T)(ikz - g.K);
@@ -1478,33 +1547,6 @@ __device__ __forceinline__ TileMode<T> tile_mode(const Geom3<T>& g, long i) {
 template <typename T>
 __device__ __forceinline__ void load3(const Fields4<T>& F, long i, cpx<T> (&x)[3]) {
   x[0] = F.c[0][i]; x[1] = F.c[1][i]; x[2] = F.c[2][i];
-}
-
-// out = -LL C (Pa + Pb)                       (tangent right-hand side)
-// out = -LL (B Pa + Pb)                       (adjoint right-hand side)
-template <typename T>
-__global__ void lin_combine(Geom3<T> g, int adjoint, Fields4<T> Pa, Fields4<T> Pb, Fields4<T> out,
-                            long len) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < len;
-       i += (long)gridDim.x * blockDim.x) {
-    const TileMode<T> m = tile_mode(g, i);
-    cpx<T> a[3], b[3], r[3];
-    load3(Pa, i, a);
-    load3(Pb, i, b);
-    if (!adjoint) {
-      cpx<T> s[3];
-      for (int c = 0; c < 3; ++c) s[c] = cpx<T>{a[c].x + b[c].x, a[c].y + b[c].y};
-      for (int c = 0; c < 3; ++c) r[c] = spec_op<T>(OP_CURL, c, s, m.kx, m.ky, m.kz, (T)0);
-    } else {
-      const T wki = wkinv(m.wk);
-      for (int c = 0; c < 3; ++c) {
-        const cpx<T> ba = spec_op<T>(OP_BS, c, a, m.kx, m.ky, m.kz, wki);
-        r[c] = cpx<T>{ba.x + b[c].x, ba.y + b[c].y};
-      }
-    }
-    const T LL = m.keep ? (T)-1 : (T)0;
-    for (int c = 0; c < 3; ++c) out.c[c][i] = cpx<T>{LL * r[c].x, LL * r[c].y};
-  }
 }
 
 // CN factor of an RK stage, (1 - q nk)/(1 + q nk) = 1 - e
@@ -1750,6 +1792,11 @@ struct Engine3D final : Engine3DBase {
   // tangent of X0 after a tangent step, valid while lin_dx is set
   Fields4<T> LX{}, LDX{};
   bool lin_dx = false;
+  // the passes' buffers over the linearised step's fields (the engine's own for
+  // the Boussinesq scheme, whose nine fields they hold) and the x-pass's resident
+  // blocks (tangent, adjoint)
+  cpx<T>*LB1 = nullptr, *LB2 = nullptr, *lin_buf = nullptr;
+  int lin_resident[2] = {1, 1};
   Fields4<T> SA{}, SB{};       // Boussinesq adjoint products: psi (i k rho) | psi u
   int c_variant = 0;           // x-pass variant chosen by the autotuner
   // pass A on packed f32x2 transforms (FP32 engine; chosen by the autotuner
@@ -1911,7 +1958,8 @@ struct Engine3D final : Engine3DBase {
     if (d_rms) cudaFree(d_rms);
     d_rms = nullptr;
     if (lin) cudaFree(lin);
-    lin = nullptr;
+    if (lin_buf) cudaFree(lin_buf);
+    lin = lin_buf = nullptr;
     d_energ = nullptr; d_umax = nullptr; d_flux = nullptr;
     pool = nullptr; stage_h = nullptr; dump = nullptr; d_status = nullptr;
   }
@@ -2202,9 +2250,9 @@ struct Engine3D final : Engine3DBase {
     const Fields4<T> none{};
     if (bous)
       return launch_k(chain, pass_a<T, N, 4, 9, 0, 3>, dim3(XT, g.Y), dim3(3 * kTileW * G), smem_a(), g,
-                      in, B1, tw, mv, d_status, full, none, 0);
+                      in, B1, tw, mv, d_status, full, none);
     return launch_k(chain, pass_a<T, N, 3, 6>, dim3(XT, g.Y), dim3(2 * kTileW * G), smem_a(), g, in, B1,
-                    tw, mv, d_status, full, none, 0);
+                    tw, mv, d_status, full, none);
   }
 
   // chain: the stream's last operation is the pass E of the previous
@@ -2410,6 +2458,11 @@ struct Engine3D final : Engine3DBase {
     return sizeof(cpx<T>) * ((size_t)no * tilew + g.n + (alias ? over + (tg - 1) * exw : tg * exw));
   }
   size_t smem_pair() const { return smem_a_nc(6); }
+  // x-pass of the linearised step: 128 threads, one copy buffer per warp, ni fields
+  size_t smem_c_lin(int ni) const {
+    const size_t L = (size_t)(128 / fft_g());
+    return sizeof(cpx<T>) * ((size_t)ni * L * g.XP + 2 * g.n + L * row_stride());
+  }
 
   template <int N>
   int lin_attrs() {
@@ -2418,17 +2471,33 @@ struct Engine3D final : Engine3DBase {
     PSG_CUDA_TRY(cudaDeviceGetAttribute(&big, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     big -= 1024;
     const bool bous = (scheme == SCHEME_BOUS_RK4);
-    const size_t need = std::max(std::max(smem_pair(), smem_e_no(3)),
-                                 bous ? std::max(smem_a_nc(5), smem_e_no(6)) : (size_t)0);
+    const size_t need = std::max(std::max(smem_pair(), std::max(smem_e_no(6), smem_c_lin(bous ? 9 : 12))),
+                                 bous ? smem_a_nc(5) : (size_t)0);
     if (need > (size_t)big) {
       psg_set_error("linearised step at grid %d needs %zu bytes of shared memory per block", g.n,
                     need);
       return PSG_ERR_UNSUPPORTED;
     }
-    PSG_CUDA_TRY(cudaFuncSetAttribute(pass_a<T, N, 6, 6, 1>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    PSG_CUDA_TRY(cudaFuncSetAttribute(pass_e<T, N, 3, SCHEME_RAW>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+#define PSG_SMEM(...) \
+    PSG_CUDA_TRY(cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, big))
+    constexpr int L = 128 / LineFFT<N, 1, T>::G;
+    int nsm = 0, occ = 0;
+    PSG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    PSG_SMEM((pass_a<T, N, 6, 9, 3>));
+    PSG_SMEM((pass_c<T, N, 9 + kLinAdj, L, 1>));
+    PSG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pass_c<T, N, 9 + kLinAdj, L, 1>, 128,
+                                                               smem_c_lin(9)));
+    lin_resident[1] = nsm * std::max(occ, 1);
+    if (!bous) {
+      PSG_SMEM((pass_a<T, N, 6, 12, 4>));
+      PSG_SMEM((pass_e<T, N, 3, SCHEME_LIN>));
+      PSG_SMEM((pass_e<T, N, 6, SCHEME_LIN>));
+      PSG_SMEM((pass_c<T, N, 12 + kLinTan, L, 1>));
+      PSG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pass_c<T, N, 12 + kLinTan, L, 1>, 128,
+                                                                 smem_c_lin(12)));
+      lin_resident[0] = nsm * std::max(occ, 1);
+    }
+#undef PSG_SMEM
     if (bous) {
       PSG_CUDA_TRY(cudaFuncSetAttribute(pass_a<T, N, 5, 7, 2>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, big));
@@ -2454,6 +2523,14 @@ struct Engine3D final : Engine3DBase {
     Fields4<T>* st[kState] = {&Zb[0], &Zb[1], &Zb[2], &Zb[3], &LA, &LN, &LS,
                               &LZ, &LK1, &LK2, &LK3, &LD, &LT, &LX, &LDX};
     const long words = ((long)kState * nc + 3 + 3 + (nc > 3 ? 6 : 0)) * box;
+    LB1 = B1;
+    LB2 = B2;
+    if (nc == 3) {
+      const long n1 = 12L * g.n * g.Y * g.XP, n2 = 12L * g.n * g.n * g.XP;
+      PSG_CUDA_TRY(cudaMalloc(&lin_buf, sizeof(cpx<T>) * (n1 + n2)));
+      LB1 = lin_buf;
+      LB2 = lin_buf + n1;
+    }
     PSG_CUDA_TRY(cudaMalloc(&lin, sizeof(cpx<T>) * words));
     PSG_CUDA_TRY(cudaMemsetAsync(lin, 0, sizeof(cpx<T>) * words, stream));
     cpx<T>* p = lin;
@@ -2468,24 +2545,43 @@ struct Engine3D final : Engine3DBase {
     return PSG_OK;
   }
 
-  // out = P(a, b) = F(-(E(op_a a) x E(op_b b))), a in pass C's u slots, b in its w slots
-  template <int N>
-  int bilinear_n(Fields4<T> b, int op_b, Fields4<T> a, int op_a, Fields4<T> out) {
-    using FG = LineFFT<N, 1, T>;
-    const dim3 blk(kTileW * FG::G), blk2(2 * kTileW * FG::G);
-    const int XT = g.XP / kTileW;
-    pass_a<T, N, 6, 6, 1><<<dim3(XT, g.Y), blk2, smem_pair(), stream>>>(
-        g, b, B1, tw, 0, d_status, nullptr, a, op_b | (op_a << 4));
-    pass_b<T, N><<<dim3(XT, N, 6), blk, smem_b(), stream>>>(g, B1, B2, tw, d_status, nullptr);
-    launch_c<N>(c_variant, (T)1 / ((T)N * (T)N * (T)N), nullptr, 6);
-    pass_d<T, N><<<dim3(XT, N, 3), blk, smem_d(), stream>>>(g, B1, B2, tw, d_status, nullptr);
+  // One right-hand side of the linearised step: the five passes over the nine
+  // (adjoint) or twelve (tangent) fields of z and x, chained like a step's.
+  // Navier-Stokes: out = N'(z) x or N'(z)^T x.  Boussinesq (adjoint): the
+  // products PA = F(-(E(z) x E(C x))), PB = F(-(E(C x) x E(B z))) themselves.
+  template <int N, bool ADJ>
+  int lin_products(Fields4<T> z, Fields4<T> x, Fields4<T> out) {
+    constexpr int G = LineFFT<N, 1, T>::G, NF = ADJ ? 9 : 12, NO = ADJ ? 6 : 3;
+    constexpr int L = 128 / G, RPW = 32 / G;
+    const dim3 blk(kTileW * G), blk2(2 * kTileW * G);
+    const int XT = g.XP / kTileW, nwt = N * N / RPW, nblk = nwt / (L / RPW);
+    const bool raw = scheme == SCHEME_BOUS_RK4;
+    int rc = launch_k(false, pass_a<T, N, 6, NF, ADJ ? 3 : 4>, dim3(XT, g.Y), blk2, smem_pair(), g, z, LB1, tw,
+                      0, d_status, nullptr, x);
+    if (rc) return rc;
+    if ((rc = launch_k(true, pass_b<T, N>, dim3(XT, N, NF), blk, smem_b(), g, LB1, LB2, tw, d_status, nullptr)))
+      return rc;
+    if ((rc = launch_k(pdl != 2, pass_c<T, N, NF + (ADJ ? kLinAdj : kLinTan), L, 1>,
+                       dim3(std::min(nblk, lin_resident[ADJ])), dim3(L * G), smem_c_lin(NF), g, LB2, LB1, tw,
+                       (T)1 / ((T)N * (T)N * (T)N), nullptr, d_status, nwt, nullptr, 0)))
+      return rc;
+    if ((rc = launch_k(true, pass_d<T, N>, dim3(XT, N, NO), blk, smem_d(), g, LB1, LB2, tw, d_status, nullptr)))
+      return rc;
     Regs<T> Rr{};
     Rr.K1 = out;
-    pass_e<T, N, 3, SCHEME_RAW><<<dim3(XT, g.Y), blk2, smem_e_no(3), stream>>>(g, B2, tw, Rr, prm, 0,
-                                                                          d_status, nullptr);
+    if (ADJ && raw) {
+      for (int q = 0; q < 3; ++q) Rr.K1.c[q] = PA.c[q];
+      Rr.K1.c[3] = PB.c[0];
+      Rr.K2.c[0] = PB.c[1];
+      Rr.K2.c[1] = PB.c[2];
+      rc = launch_k(true, pass_e<T, N, 6, SCHEME_RAW>, dim3(XT, g.Y), blk2, smem_e_no(6), g, LB2, tw, Rr, prm,
+                    0, d_status, nullptr);
+    } else {
+      rc = launch_k(true, pass_e<T, N, NO, SCHEME_LIN>, dim3(XT, g.Y), blk2, smem_e_no(NO), g, LB2, tw, Rr, prm,
+                    0, d_status, nullptr);
+    }
     launches += 5;
-    PSG_CUDA_TRY(cudaGetLastError());
-    return PSG_OK;
+    return rc;
   }
   // SA, SB <- the Boussinesq adjoint's scalar products of psi = E(x_rho) with
   // E(i k z_rho) and E(B z_w)
@@ -2497,7 +2593,7 @@ struct Engine3D final : Engine3DBase {
     Fields4<T> psi{};
     psi.c[0] = x.c[3];
     pass_a<T, N, 5, 7, 2><<<dim3(XT, g.Y), blk2, smem_a_nc(5), stream>>>(g, z, B1, tw, 0, d_status,
-                                                                         nullptr, psi, 0);
+                                                                         nullptr, psi);
     pass_b<T, N><<<dim3(XT, N, 7), blk, smem_b(), stream>>>(g, B1, B2, tw, d_status, nullptr);
     launch_c<N>(c_variant, (T)1 / ((T)N * (T)N * (T)N), nullptr, 7);
     pass_d<T, N><<<dim3(XT, N, 6), blk, smem_d(), stream>>>(g, B1, B2, tw, d_status, nullptr);
@@ -2528,25 +2624,12 @@ struct Engine3D final : Engine3DBase {
     return t;
   }
 
-  int bilinear(Fields4<T> b, int op_b, Fields4<T> a, int op_a, Fields4<T> out) {
-    return bilinear_n<NN>(b, op_b, a, op_a, out);
-  }
-
   // out = N'(z) x (tangent) or N'(z)^T x (adjoint)
   int lin_rhs(int adjoint, Fields4<T> z, Fields4<T> x, Fields4<T> out) {
     int rc;
     if (scheme == SCHEME_BOUS_RK4) return lin_rhs_bous(adjoint, z, x, out);
-    if (!adjoint) {
-      if ((rc = bilinear(z, OP_ID, x, OP_BS, PA))) return rc;  // F(-(E(B x) x E(z)))
-      if ((rc = bilinear(x, OP_ID, z, OP_BS, PB))) return rc;  // F(-(E(B z) x E(x)))
-    } else {
-      if ((rc = bilinear(x, OP_CURL, z, OP_ID, PA))) return rc;  // F(-(E(z) x E(C x)))
-      if ((rc = bilinear(z, OP_BS, x, OP_CURL, PB))) return rc;  // F(-(E(C x) x E(B z)))
-    }
-    lin_combine<T><<<592, 256, 0, stream>>>(g, adjoint, PA, PB, out, box);
-    ++launches;
-    PSG_CUDA_TRY(cudaGetLastError());
-    return PSG_OK;
+    rc = adjoint ? lin_products<NN, true>(z, x, out) : lin_products<NN, false>(z, x, out);
+    return rc;
   }
 
   // Boussinesq: the tangent as the central difference of the engine's own
@@ -2582,8 +2665,7 @@ struct Engine3D final : Engine3DBase {
       PSG_CUDA_TRY(cudaGetLastError());
       return PSG_OK;
     }
-    if ((rc = bilinear(x, OP_CURL, z, OP_ID, PA))) return rc;  // F(-(E(z) x E(C x)))
-    if ((rc = bilinear(z, OP_BS, x, OP_CURL, PB))) return rc;  // F(-(E(C x) x E(B z)))
+    if ((rc = lin_products<NN, true>(z, x, out))) return rc;  // PA, PB
     if ((rc = scale_products(z, x))) return rc;
     bous_adj_combine<T><<<592, 256, 0, stream>>>(g, prm.ri, prm.sinth, prm.costh, PA, PB, SA, SB,
                                                  x, out, box);
