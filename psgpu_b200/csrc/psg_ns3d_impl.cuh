@@ -223,9 +223,22 @@ __device__ __forceinline__ bool a_stage(const Geom3<T>& g, Src src_comp, const c
   return true;
 }
 
+// Lane groups of pass A over nf fields: grids up to 64^3 are a chain of short
+// passes, so every field gets a group (one transform deep; at most 8 for the
+// block size); larger grids fill the SMs with two (three for the nine Boussinesq
+// fields: no round is left half idle).
+template <int N>
+constexpr int a_groups(int nf) {
+  return N <= 64 ? (nf == 12 ? 6 : nf) : nf == 9 ? 3 : 2;
+}
+// the same with the six staged vectors of the linearised step
+template <int N>
+constexpr int lin_groups(int nf) {
+  return N <= 64 ? a_groups<N>(nf) : 2;
+}
 template <typename T, int N, int NC, int NF, int MODE = 0, int NG = 2>
 __global__ void __launch_bounds__(NG * kTileW * LineFFT<N, 1, T>::G,
-                                  sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : (NG == 2 ? 3 : 2))
+                                  N <= 64 ? 1 : sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : (NG == 2 ? 3 : 2))
 pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __restrict__ tw,
        int mask_vel, int* status, const int* __restrict__ full, Fields4<T> in2 = Fields4<T>{}) {
   using F = LineFFT<N, +1, T>;
@@ -946,6 +959,10 @@ pass_d(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
   }
 }
 
+}  // namespace psg
+#include "psg_plane.cuh"
+namespace psg {
+
 // ---------------------------------------------------------------------------
 // pass E: z-forward of the NO fields of one (xt, ky) tile, then the spectral
 // finish and the scheme update for every mode of the tile.
@@ -1183,8 +1200,12 @@ struct GroupSync {
 // Pass E runs 2 W G threads: for three fields both halves transform the tile,
 // for more the first half alone (named barriers of their own), then all of
 // them do the update, whose state loads are what the pass waits on.
+// Grids up to 64^3 take NO W G threads instead and transform every field at once.
+template <int N>
+constexpr int e_groups(int no) { return N <= 64 ? no : 2; }
 template <typename T, int N, int NO, int SCHEME>
-__global__ void __launch_bounds__(2 * kTileW * LineFFT<N, 1, T>::G, sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : 3)
+__global__ void __launch_bounds__(e_groups<N>(NO) * kTileW * LineFFT<N, 1, T>::G,
+                                  N <= 64 ? 1 : sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : 3)
 pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw, Regs<T> R,
        StepParams<T> p, int stage, int* status, const int* __restrict__ full) {
   using F = LineFFT<N, -1, T>;
@@ -1204,7 +1225,7 @@ pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw,
   constexpr int R0 = N - Y;  // first output row
   cpx<T>* s_in = reinterpret_cast<cpx<T>*>(smem_raw);  // [NO][N][W] (+ pad)
   cpx<T>* s_tw = s_in + NO * N * W + (ALIAS ? OVER : 0);
-  constexpr int TG = (NO == 3) ? 2 : 1;                // transform groups
+  constexpr int TG = N <= 64 ? NO : (NO == 3) ? 2 : 1;  // transform groups
   cpx<T>* s_ex = s_tw + N;  // without ALIAS: the first group's; then the second's
   const int tid = threadIdx.x, nth = blockDim.x, c = tid % W;
   const int xt = blockIdx.x, iky = blockIdx.y;
@@ -1253,7 +1274,7 @@ pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw,
 #pragma unroll
         for (int e = 0; e < F::E; ++e) v[e] = s_in[(f * N + F::in_index(tl, e)) * W + c];
         const NamedSync gs{1 + tg, W * F::G};
-        cpx<T>* exb = (tg == 0) ? (ALIAS ? s_in + f * N * W : s_ex) : s_ex + (ALIAS ? 0 : W * SX);
+        cpx<T>* exb = (tg == 0 && ALIAS) ? s_in + f * N * W : s_ex + (tg - (ALIAS ? 1 : 0)) * W * SX;
         if (ALIAS && tg == 0) gs();  // every input read before the exchange reuses them
         F::run(v, tl, s_tw, exb + c * SX, gs);
 #pragma unroll
@@ -1805,6 +1826,7 @@ struct Engine3D final : Engine3DBase {
   float a_ms[2] = {-1.f, -1.f};
   int c_resident[16] = {1, 1, 1, 1};  // resident blocks of each x-pass variant
   float c_ms[16] = {};                 // autotuner timings (ms per launch)
+  size_t plane_smem_max = 0;   // shared memory the plane kernel may use
   long launches = 0;
   // optional per-pass timing with CUDA events recorded between the passes
   bool profiling = false;
@@ -1854,7 +1876,7 @@ struct Engine3D final : Engine3DBase {
   // dynamic shared memory of each pass (must match the kernels' carve-up)
   // pass A runs three groups of W x G threads for the nine Boussinesq fields
   // (three rounds, none idle) and two for the six Navier-Stokes fields
-  int groups_a() const { return nc == 4 ? 3 : 2; }
+  int groups_a() const { return a_groups<NN>(nc == 4 ? 9 : 6); }
   size_t smem_a() const { return smem_a_nc(nc, groups_a()); }
   // passes B and D: one area for the staged tile and then the exchange; twiddles
   size_t smem_b() const {
@@ -1978,8 +2000,10 @@ struct Engine3D final : Engine3DBase {
         return PSG_ERR_UNSUPPORTED;
       }
 #define PSG_SMEM(kern) PSG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, big))
-    PSG_SMEM((pass_a<T, N, 3, 6>));
-    PSG_SMEM((pass_a<T, N, 4, 9, 0, 3>));
+    plane_smem_max = (size_t)big;
+    if (int rc = scheme == SCHEME_BOUS_RK4 ? plane_attrs<9>() : plane_attrs<6>()) return rc;
+    PSG_SMEM((pass_a<T, N, 3, 6, 0, a_groups<N>(6)>));
+    PSG_SMEM((pass_a<T, N, 4, 9, 0, a_groups<N>(9)>));
     if constexpr (sizeof(T) == 4) {
       a_pk_ok = smem_a_pk_n<N>(nc) <= (size_t)big;
       if (a_pk_ok) {
@@ -2231,6 +2255,55 @@ struct Engine3D final : Engine3DBase {
     return fresh ? d_full + slot : nullptr;
   }
 
+  // threads of the plane kernel over NF fields: its widest phase's lines, whole
+  // warps, fewer where the exchange space would not fit; 0 where it is not built
+  // or does not fit at all
+  template <int NF>
+  int plane_threads() const {
+    if constexpr (PlaneShape<NN>::built(NF, sizeof(T))) {
+      using PL = Plane<T, NN, NF>;
+      int nt = std::min(kPlaneThreads, (PL::lines() * PL::G + 31) / 32 * 32);
+      while (nt >= 64 && PL::smem(nt) > plane_smem_max) nt -= 32;
+      return nt >= 64 ? nt : 0;
+    }
+    return 0;
+  }
+  template <int NF>
+  int plane_attrs() {
+    if constexpr (PlaneShape<NN>::built(NF, sizeof(T)))
+      PSG_CUDA_TRY(cudaFuncSetAttribute(pass_bcd<T, NN, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)plane_smem_max));
+    return PSG_OK;
+  }
+  // passes B, C and D as one kernel
+  template <int NF>
+  int launch_plane(const cpx<T>* in, cpx<T>* out, const int* full, T* dp = nullptr) {
+    if constexpr (PlaneShape<NN>::built(NF, sizeof(T))) {
+      using PL = Plane<T, NN, NF>;
+      const int nt = plane_threads<NF>();
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(PL::CS * NN);
+      cfg.blockDim = dim3(nt);
+      cfg.dynamicSmemBytes = PL::smem(nt);
+      cfg.stream = stream;
+      cudaLaunchAttribute at[2];
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = PL::CS;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      if (pdl) {
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
+      }
+      const T scale = (T)1 / ((T)NN * (T)NN * (T)NN);
+      PSG_CUDA_TRY(cudaLaunchKernelEx(&cfg, pass_bcd<T, NN, NF>, in, out, (const cpx<T>*)tw, scale, full, dp,
+                                      (dump_mode & 2) ? 6 : 3));
+    }
+    return PSG_OK;
+  }
+
   // one right-hand-side evaluation followed by the stage update
   // pass A of the step's right-hand side, scalar or on packed transforms
   template <int N>
@@ -2249,9 +2322,9 @@ struct Engine3D final : Engine3DBase {
     }
     const Fields4<T> none{};
     if (bous)
-      return launch_k(chain, pass_a<T, N, 4, 9, 0, 3>, dim3(XT, g.Y), dim3(3 * kTileW * G), smem_a(), g,
+      return launch_k(chain, pass_a<T, N, 4, 9, 0, a_groups<N>(9)>, dim3(XT, g.Y), dim3(groups_a() * kTileW * G), smem_a(), g,
                       in, B1, tw, mv, d_status, full, none);
-    return launch_k(chain, pass_a<T, N, 3, 6>, dim3(XT, g.Y), dim3(2 * kTileW * G), smem_a(), g, in, B1,
+    return launch_k(chain, pass_a<T, N, 3, 6, 0, a_groups<N>(6)>, dim3(XT, g.Y), dim3(groups_a() * kTileW * G), smem_a(), g, in, B1,
                     tw, mv, d_status, full, none);
   }
 
@@ -2267,11 +2340,21 @@ struct Engine3D final : Engine3DBase {
     const int mv = first_rhs;
     first_rhs = 0;
     mark(-1);
-    const dim3 blk2(2 * kTileW * G);
+    const dim3 blk_e(e_groups<N>(nfo) * kTileW * G);
     const int* full = full_flag(stage);
     int rc = launch_a<N>(chain, a_pk, in, mv, full);
     if (rc) return rc;
     mark(0);
+    // the plane kernel where it is built; passes of their own for the per-pass
+    // events, for max |u| and, at 64^3, for the physical fields
+    const bool plane = (scheme == SCHEME_BOUS_RK4 ? plane_threads<9>() : plane_threads<6>()) > 0 && !profiling &&
+                       !want_umax && (!want_dump || N <= 32);
+    if (plane) {
+      T* kept = want_dump ? dump : nullptr;
+      rc = scheme == SCHEME_BOUS_RK4 ? launch_plane<9>(B1, B2, full, kept) : launch_plane<6>(B1, B2, full, kept);
+      if (rc) return rc;
+      launches -= 2;
+    } else {
     if ((rc = launch_k(true, pass_b<T, N>, dim3(XT, N, nfi), blk, smem_b(), g, B1, B2, tw, d_status, full)))
       return rc;
     mark(1);
@@ -2286,22 +2369,23 @@ struct Engine3D final : Engine3DBase {
     if ((rc = launch_k(true, pass_d<T, N>, dim3(XT, N, nfo), blk, smem_d(), g, B1, B2, tw, d_status, full)))
       return rc;
     mark(3);
+    }
     const dim3 ge(XT, g.Y);
     switch (scheme) {
       case SCHEME_NS_HEUN:
-        rc = launch_k(true, pass_e<T, N, 3, SCHEME_NS_HEUN>, ge, blk2, smem_e(), g, B2, tw, R, prm,
+        rc = launch_k(true, pass_e<T, N, 3, SCHEME_NS_HEUN>, ge, blk_e, smem_e(), g, B2, tw, R, prm,
                       stage, d_status, full);
         break;
       case SCHEME_EULER_HEUN:
-        rc = launch_k(true, pass_e<T, N, 3, SCHEME_EULER_HEUN>, ge, blk2, smem_e(), g, B2, tw, R, prm,
+        rc = launch_k(true, pass_e<T, N, 3, SCHEME_EULER_HEUN>, ge, blk_e, smem_e(), g, B2, tw, R, prm,
                       stage, d_status, full);
         break;
       case SCHEME_NS_RK4:
-        rc = launch_k(true, pass_e<T, N, 3, SCHEME_NS_RK4>, ge, blk2, smem_e(), g, B2, tw, R, prm,
+        rc = launch_k(true, pass_e<T, N, 3, SCHEME_NS_RK4>, ge, blk_e, smem_e(), g, B2, tw, R, prm,
                       stage, d_status, full);
         break;
       default:
-        rc = launch_k(true, pass_e<T, N, 4, SCHEME_BOUS_RK4>, ge, blk2, smem_e(), g, B2, tw, R, prm,
+        rc = launch_k(true, pass_e<T, N, 4, SCHEME_BOUS_RK4>, ge, blk_e, smem_e(), g, B2, tw, R, prm,
                       stage, d_status, full);
     }
     if (rc) return rc;
@@ -2454,10 +2538,10 @@ struct Engine3D final : Engine3DBase {
     const long exw = (long)kTileW * col_stride(), tilew = (long)g.n * kTileW;
     const long over = exw > tilew ? exw - tilew : 0;
     const bool alias = over <= (long)(g.n - g.Y) * kTileW;
-    const int tg = (no == 3) ? 2 : 1;  // transform groups (one exchange area each)
+    const int tg = NN <= 64 ? no : (no == 3) ? 2 : 1;  // transform groups (one exchange area each)
     return sizeof(cpx<T>) * ((size_t)no * tilew + g.n + (alias ? over + (tg - 1) * exw : tg * exw));
   }
-  size_t smem_pair() const { return smem_a_nc(6); }
+  size_t smem_pair() const { return smem_a_nc(6, std::max(lin_groups<NN>(9), lin_groups<NN>(12))); }
   // x-pass of the linearised step: 128 threads, one copy buffer per warp, ni fields
   size_t smem_c_lin(int ni) const {
     const size_t L = (size_t)(128 / fft_g());
@@ -2483,13 +2567,16 @@ struct Engine3D final : Engine3DBase {
     constexpr int L = 128 / LineFFT<N, 1, T>::G;
     int nsm = 0, occ = 0;
     PSG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    PSG_SMEM((pass_a<T, N, 6, 9, 3>));
+    if (int rc = plane_attrs<9 + kLinAdj>()) return rc;
+    if (!bous)
+      if (int rc = plane_attrs<12 + kLinTan>()) return rc;
+    PSG_SMEM((pass_a<T, N, 6, 9, 3, lin_groups<N>(9)>));
     PSG_SMEM((pass_c<T, N, 9 + kLinAdj, L, 1>));
     PSG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pass_c<T, N, 9 + kLinAdj, L, 1>, 128,
                                                                smem_c_lin(9)));
     lin_resident[1] = nsm * std::max(occ, 1);
     if (!bous) {
-      PSG_SMEM((pass_a<T, N, 6, 12, 4>));
+      PSG_SMEM((pass_a<T, N, 6, 12, 4, lin_groups<N>(12)>));
       PSG_SMEM((pass_e<T, N, 3, SCHEME_LIN>));
       PSG_SMEM((pass_e<T, N, 6, SCHEME_LIN>));
       PSG_SMEM((pass_c<T, N, 12 + kLinTan, L, 1>));
@@ -2553,12 +2640,18 @@ struct Engine3D final : Engine3DBase {
   int lin_products(Fields4<T> z, Fields4<T> x, Fields4<T> out) {
     constexpr int G = LineFFT<N, 1, T>::G, NF = ADJ ? 9 : 12, NO = ADJ ? 6 : 3;
     constexpr int L = 128 / G, RPW = 32 / G;
-    const dim3 blk(kTileW * G), blk2(2 * kTileW * G);
+    const dim3 blk(kTileW * G), blk_e(e_groups<N>(NO) * kTileW * G);
     const int XT = g.XP / kTileW, nwt = N * N / RPW, nblk = nwt / (L / RPW);
     const bool raw = scheme == SCHEME_BOUS_RK4;
-    int rc = launch_k(false, pass_a<T, N, 6, NF, ADJ ? 3 : 4>, dim3(XT, g.Y), blk2, smem_pair(), g, z, LB1, tw,
+    int rc = launch_k(false, pass_a<T, N, 6, NF, ADJ ? 3 : 4, lin_groups<N>(NF)>, dim3(XT, g.Y),
+                      dim3(lin_groups<N>(NF) * kTileW * G), smem_a_nc(6, lin_groups<N>(NF)), g, z, LB1, tw,
                       0, d_status, nullptr, x);
     if (rc) return rc;
+    if (plane_threads<NF + (ADJ ? kLinAdj : kLinTan)>() > 0) {
+      rc = launch_plane<NF + (ADJ ? kLinAdj : kLinTan)>(LB1, LB2, nullptr);
+      if (rc) return rc;
+      launches -= 2;
+    } else {
     if ((rc = launch_k(true, pass_b<T, N>, dim3(XT, N, NF), blk, smem_b(), g, LB1, LB2, tw, d_status, nullptr)))
       return rc;
     if ((rc = launch_k(pdl != 2, pass_c<T, N, NF + (ADJ ? kLinAdj : kLinTan), L, 1>,
@@ -2567,6 +2660,7 @@ struct Engine3D final : Engine3DBase {
       return rc;
     if ((rc = launch_k(true, pass_d<T, N>, dim3(XT, N, NO), blk, smem_d(), g, LB1, LB2, tw, d_status, nullptr)))
       return rc;
+    }
     Regs<T> Rr{};
     Rr.K1 = out;
     if (ADJ && raw) {
@@ -2574,10 +2668,10 @@ struct Engine3D final : Engine3DBase {
       Rr.K1.c[3] = PB.c[0];
       Rr.K2.c[0] = PB.c[1];
       Rr.K2.c[1] = PB.c[2];
-      rc = launch_k(true, pass_e<T, N, 6, SCHEME_RAW>, dim3(XT, g.Y), blk2, smem_e_no(6), g, LB2, tw, Rr, prm,
+      rc = launch_k(true, pass_e<T, N, 6, SCHEME_RAW>, dim3(XT, g.Y), blk_e, smem_e_no(6), g, LB2, tw, Rr, prm,
                     0, d_status, nullptr);
     } else {
-      rc = launch_k(true, pass_e<T, N, NO, SCHEME_LIN>, dim3(XT, g.Y), blk2, smem_e_no(NO), g, LB2, tw, Rr, prm,
+      rc = launch_k(true, pass_e<T, N, NO, SCHEME_LIN>, dim3(XT, g.Y), blk_e, smem_e_no(NO), g, LB2, tw, Rr, prm,
                     0, d_status, nullptr);
     }
     launches += 5;
@@ -2600,7 +2694,7 @@ struct Engine3D final : Engine3DBase {
     Regs<T> Rr{};
     Rr.K1 = SA;
     Rr.K2 = SB;
-    pass_e<T, N, 6, SCHEME_RAW><<<dim3(XT, g.Y), blk2, smem_e_no(6), stream>>>(g, B2, tw, Rr, prm, 0,
+    pass_e<T, N, 6, SCHEME_RAW><<<dim3(XT, g.Y), e_groups<N>(6) * kTileW * FG::G, smem_e_no(6), stream>>>(g, B2, tw, Rr, prm, 0,
                                                                               d_status, nullptr);
     launches += 5;
     PSG_CUDA_TRY(cudaGetLastError());
