@@ -169,4 +169,152 @@ struct LineFFT {
   }
 };
 
+// ---------------------------------------------------------------------------
+// LineFFTM: LineFFT's decomposition, distributions and exchange with the
+// twiddles of the second step merged into its butterflies.
+//
+// With z_k = w_N^{k2 + R2 k} the second step's outputs are the polynomial
+// sum_n y_n z^n at z = z_0 .. z_{R1-1}, and a radix-2 decimation in time evaluates
+// it with the factors tau_{m,j} = z_j^{R1/m} (block size m, j < m/2), so that no
+// multiplication stands apart from a butterfly.  tau_{m, j + m/4} = +-i tau_{m,j}:
+// R1/2 table entries per k2 (eight 16-byte loads per 16 points instead of 16).
+// A butterfly a +- tau b is four multiply-adds for the sum and two for the
+// difference, 2 a - (a + tau b); the first step's constant factors go the same
+// way.  Per 256-point line and lane: 340 FP instructions instead of 396; the
+// x-pass, bound by its arithmetic, went from 116 to 105 us (256^3 FP32), 229 to 184
+// (256^3 FP64) and 41 to 35 (128^3 FP64).  The 2D search's small grids and the
+// allocation-free step keep LineFFT.
+// ---------------------------------------------------------------------------
+
+// a, b <- a + (c + i s) b, a - (c + i s) b
+template <typename T>
+__device__ __forceinline__ void bfly(cpx<T>& a, cpx<T>& b, T c, T s) {
+  const cpx<T> p = cpx<T>{fma(-s, b.y, fma(c, b.x, a.x)), fma(s, b.x, fma(c, b.y, a.y))};
+  b = cpx<T>{fma((T)2, a.x, -p.x), fma((T)2, a.y, -p.y)};
+  a = p;
+}
+
+// v[bit-reversed i] = x[i]; the index loops unroll with the caller's (a function
+// returning the index did not for R = 16, which put the arrays in local memory)
+template <int R, typename V>
+__device__ __forceinline__ void bit_reversed(const V (&x)[R], V (&v)[R]) {
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    int r = 0;
+#pragma unroll
+    for (int b = 1, q = R >> 1; b < R; b <<= 1, q >>= 1)
+      if (i & b) r |= q;
+    v[r] = x[i];
+  }
+}
+
+// in-register R-point DFT, natural order in and out
+// blocks of LEN points and larger (a template per level: the level loop of a
+// 16-point transform did not unroll, which put the array in local memory)
+template <int R, int LEN, int SIGN, typename T>
+__device__ __forceinline__ void dft_dit_level(cpx<T> (&v)[R]) {
+  constexpr int half = LEN >> 1;
+#pragma unroll
+  for (int s = 0; s < R; s += LEN) {
+#pragma unroll
+    for (int j = 0; j < half; ++j) {
+      cpx<T>&a = v[s + j], &b = v[s + j + half];
+      const int m = j * (32 / LEN);
+      if (m == 0) {
+        const cpx<T> d = cpx<T>{a.x - b.x, a.y - b.y};
+        a = cpx<T>{a.x + b.x, a.y + b.y};
+        b = d;
+      } else if (m == 8) {  // SIGN i b
+        const cpx<T> t = SIGN < 0 ? cpx<T>{b.y, -b.x} : cpx<T>{-b.y, b.x};
+        b = cpx<T>{a.x - t.x, a.y - t.y};
+        a = cpx<T>{a.x + t.x, a.y + t.y};
+      } else {
+        bfly(a, b, Omega32<T>::c(m), (T)SIGN * Omega32<T>::s(m));
+      }
+    }
+  }
+  if constexpr (LEN < R) dft_dit_level<R, 2 * LEN, SIGN>(v);
+}
+
+template <int R, int SIGN, typename T>
+__device__ __forceinline__ void dft_dit(cpx<T> (&x)[R]) {
+  cpx<T> v[R];
+  bit_reversed<R>(x, v);
+  dft_dit_level<R, 2, SIGN>(v);
+#pragma unroll
+  for (int i = 0; i < R; ++i) x[i] = v[i];
+}
+
+// the R-point step with merged twiddles; tw: this line's tau entries, `stride` apart
+template <int R, int LEN, int SIGN, typename T>
+__device__ __forceinline__ void dft_tau_level(cpx<T> (&v)[R], const cpx<T>* tw, int stride) {
+  constexpr int half = LEN >> 1, quarter = LEN >> 2, nt = quarter > 0 ? quarter : 1;
+#pragma unroll
+  for (int j = 0; j < nt; ++j) {
+    cpx<T> t = tw[(quarter + j) * stride];
+    if (SIGN > 0) t.y = -t.y;
+#pragma unroll
+    for (int s = 0; s < R; s += LEN) {
+      bfly(v[s + j], v[s + j + half], t.x, t.y);
+      if (quarter > 0)  // times SIGN i
+        bfly(v[s + j + quarter], v[s + j + quarter + half], SIGN < 0 ? t.y : -t.y, SIGN < 0 ? -t.x : t.x);
+    }
+  }
+  if constexpr (LEN < R) dft_tau_level<R, 2 * LEN, SIGN>(v, tw, stride);
+}
+
+template <int R, int SIGN, typename T>
+__device__ __forceinline__ void dft_tau(cpx<T> (&x)[R], const cpx<T>* tw, int stride) {
+  cpx<T> v[R];
+  bit_reversed<R>(x, v);
+  dft_tau_level<R, 2, SIGN>(v, tw, stride);
+#pragma unroll
+  for (int i = 0; i < R; ++i) x[i] = v[i];
+}
+
+template <int N, int SIGN, typename T, bool SWAP = false>
+struct LineFFTM : LineFFT<N, SIGN, T, SWAP> {
+  using L = LineFFT<N, SIGN, T, SWAP>;
+  static constexpr int R1 = L::R1, R2 = L::R2, G = L::G, E = L::E, A = L::A, B = L::B;
+
+  // tau table: TW[i * R2 + k2], i < R1/2 (entry 0: block size 2; len/4 + j: size len);
+  // N entries are reserved, the second half is unused
+  static void host_table(cpx<T>* out) {
+    for (int i = 0; i < N; ++i) out[i] = cpx<T>{(T)0, (T)0};
+    for (int len = 2; len <= R1; len <<= 1) {
+      const int q = len / 4, nt = q > 0 ? q : 1;
+      for (int j = 0; j < nt; ++j)
+        for (int k2 = 0; k2 < R2; ++k2) {
+          const double a = -2.0 * 3.14159265358979323846 * (double)((R1 / len) * (k2 + R2 * j)) / (double)N;
+          out[(q + j) * R2 + k2] = cpx<T>{(T)cos(a), (T)sin(a)};
+        }
+    }
+  }
+
+  template <typename Sync>
+  static __device__ __forceinline__ void run(cpx<T> (&v)[E], int g, const cpx<T>* tw, cpx<T>* ex, Sync sync) {
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+      cpx<T> w[R2];
+#pragma unroll
+      for (int n2 = 0; n2 < R2; ++n2) w[n2] = v[a * R2 + n2];
+      dft_dit<R2, SIGN>(w);
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2) ex[k2 * (R1 + 1) + g + G * a] = w[k2];
+    }
+    sync();
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      cpx<T> w[R1];
+      const int k2 = g + G * b;
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) w[n1] = ex[k2 * (R1 + 1) + n1];
+      dft_tau<R1, SIGN>(w, tw + k2, R2);
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) v[b * R1 + k1] = w[k1];
+    }
+    sync();  // `ex` may be rewritten by the next call
+  }
+};
+
 }  // namespace psg

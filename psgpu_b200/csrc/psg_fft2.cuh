@@ -194,4 +194,150 @@ struct LineFFT2 {
   }
 };
 
+// LineFFTM (merged twiddles) for two lines at once
+__device__ __forceinline__ void pbfly(Pk& a, Pk& b, float c, float s) {
+  const float2 px = pfma(b.im, psplat(-s), pfma(b.re, psplat(c), a.re));
+  const float2 py = pfma(b.re, psplat(s), pfma(b.im, psplat(c), a.im));
+  b = Pk{pfma(a.re, psplat(2.f), make_float2(-px.x, -px.y)), pfma(a.im, psplat(2.f), make_float2(-py.x, -py.y))};
+  a = Pk{px, py};
+}
+
+template <int R, int LEN, int SIGN>
+__device__ __forceinline__ void pdft_dit_level(Pk (&v)[R]) {
+  constexpr int half = LEN >> 1;
+#pragma unroll
+  for (int s = 0; s < R; s += LEN) {
+#pragma unroll
+    for (int j = 0; j < half; ++j) {
+      Pk&a = v[s + j], &b = v[s + j + half];
+      const int m = j * (32 / LEN);
+      if (m == 0) {
+        const Pk d{psub(a.re, b.re), psub(a.im, b.im)};
+        a = Pk{padd(a.re, b.re), padd(a.im, b.im)};
+        b = d;
+      } else if (m == 8) {  // SIGN i b
+        const Pk p = SIGN < 0 ? Pk{padd(a.re, b.im), psub(a.im, b.re)} : Pk{psub(a.re, b.im), padd(a.im, b.re)};
+        b = SIGN < 0 ? Pk{psub(a.re, b.im), padd(a.im, b.re)} : Pk{padd(a.re, b.im), psub(a.im, b.re)};
+        a = p;
+      } else {
+        pbfly(a, b, Omega32<float>::c(m), (float)SIGN * Omega32<float>::s(m));
+      }
+    }
+  }
+  if constexpr (LEN < R) pdft_dit_level<R, 2 * LEN, SIGN>(v);
+}
+
+template <int R, int SIGN>
+__device__ __forceinline__ void pdft_dit(Pk (&x)[R]) {
+  Pk v[R];
+  bit_reversed<R>(x, v);
+  pdft_dit_level<R, 2, SIGN>(v);
+#pragma unroll
+  for (int i = 0; i < R; ++i) x[i] = v[i];
+}
+
+template <int R, int LEN, int SIGN>
+__device__ __forceinline__ void pdft_tau_level(Pk (&v)[R], const cpx<float>* tw, int stride) {
+  constexpr int half = LEN >> 1, quarter = LEN >> 2, nt = quarter > 0 ? quarter : 1;
+#pragma unroll
+  for (int j = 0; j < nt; ++j) {
+    cpx<float> t = tw[(quarter + j) * stride];
+    if (SIGN > 0) t.y = -t.y;
+#pragma unroll
+    for (int s = 0; s < R; s += LEN) {
+      pbfly(v[s + j], v[s + j + half], t.x, t.y);
+      if (quarter > 0)  // times SIGN i
+        pbfly(v[s + j + quarter], v[s + j + quarter + half], SIGN < 0 ? t.y : -t.y, SIGN < 0 ? -t.x : t.x);
+    }
+  }
+  if constexpr (LEN < R) pdft_tau_level<R, 2 * LEN, SIGN>(v, tw, stride);
+}
+
+template <int R, int SIGN>
+__device__ __forceinline__ void pdft_tau(Pk (&x)[R], const cpx<float>* tw, int stride) {
+  Pk v[R];
+  bit_reversed<R>(x, v);
+  pdft_tau_level<R, 2, SIGN>(v, tw, stride);
+#pragma unroll
+  for (int i = 0; i < R; ++i) x[i] = v[i];
+}
+
+template <int N, int SIGN, bool SWAP = false>
+struct LineFFT2M {
+  using P = LineFFTM<N, SIGN, float, SWAP>;
+  static constexpr int R1 = P::R1, R2 = P::R2, G = P::G, E = P::E, A = P::A, B = P::B;
+  static constexpr int SMEM = P::SMEM;
+
+  template <typename Sync>
+  static __device__ __forceinline__ void run(Pk (&v)[E], int g, const cpx<float>* tw, float4* ex, Sync sync) {
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+      Pk w[R2];
+#pragma unroll
+      for (int n2 = 0; n2 < R2; ++n2) w[n2] = v[a * R2 + n2];
+      pdft_dit<R2, SIGN>(w);
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2)
+        ex[k2 * (R1 + 1) + g + G * a] = make_float4(w[k2].re.x, w[k2].re.y, w[k2].im.x, w[k2].im.y);
+    }
+    sync();
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      Pk w[R1];
+      const int k2 = g + G * b;
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) {
+        const float4 q = ex[k2 * (R1 + 1) + n1];
+        w[n1] = Pk{make_float2(q.x, q.y), make_float2(q.z, q.w)};
+      }
+      pdft_tau<R1, SIGN>(w, tw + k2, R2);
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) v[b * R1 + k1] = w[k1];
+    }
+    sync();
+  }
+
+  // with an exchange buffer of 8-byte entries: the real and the imaginary parts
+  // cross it one after the other
+  template <typename Sync>
+  static __device__ __forceinline__ void run(Pk (&v)[E], int g, const cpx<float>* tw, float2* ex, Sync sync) {
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+      Pk w[R2];
+#pragma unroll
+      for (int n2 = 0; n2 < R2; ++n2) w[n2] = v[a * R2 + n2];
+      pdft_dit<R2, SIGN>(w);
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2) v[a * R2 + k2] = w[k2];
+    }
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+#pragma unroll
+      for (int a = 0; a < A; ++a)
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2)
+          ex[k2 * (R1 + 1) + g + G * a] = part == 0 ? v[a * R2 + k2].re : v[a * R2 + k2].im;
+      sync();
+#pragma unroll
+      for (int b = 0; b < B; ++b)
+#pragma unroll
+        for (int n1 = 0; n1 < R1; ++n1) {
+          const float2 q = ex[(g + G * b) * (R1 + 1) + n1];
+          if (part == 0) v[b * R1 + n1].re = q;
+          else v[b * R1 + n1].im = q;
+        }
+      sync();
+    }
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      Pk w[R1];
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) w[n1] = v[b * R1 + n1];
+      pdft_tau<R1, SIGN>(w, tw + g + G * b, R2);
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) v[b * R1 + k1] = w[k1];
+    }
+  }
+};
+
 }  // namespace psg

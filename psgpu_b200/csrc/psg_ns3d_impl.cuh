@@ -237,11 +237,11 @@ constexpr int lin_groups(int nf) {
   return N <= 64 ? a_groups<N>(nf) : 2;
 }
 template <typename T, int N, int NC, int NF, int MODE = 0, int NG = 2>
-__global__ void __launch_bounds__(NG * kTileW * LineFFT<N, 1, T>::G,
+__global__ void __launch_bounds__(NG * kTileW * LineFFTM<N, 1, T>::G,
                                   N <= 64 ? 1 : sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : (NG == 2 ? 3 : 2))
 pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __restrict__ tw,
        int mask_vel, int* status, const int* __restrict__ full, Fields4<T> in2 = Fields4<T>{}) {
-  using F = LineFFT<N, +1, T>;
+  using F = LineFFTM<N, +1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
   constexpr int Y = Box<N>::Y, K = Box<N>::K, XT = Box<N>::XT;
@@ -344,12 +344,12 @@ pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __rest
 // the pair's values side by side (16-byte words, row stride odd mod 8 so that
 // the eight columns of a quarter warp fall on distinct bank groups).
 template <int N, int NC, int NF>
-__global__ void __launch_bounds__(kTileW * LineFFT<N, 1, float>::G, 3)
+__global__ void __launch_bounds__(kTileW * LineFFTM<N, 1, float>::G, 3)
 pass_a_pk(Geom3<float> g, Fields4<float> in, cpx<float>* __restrict__ out,
           const cpx<float>* __restrict__ tw, int mask_vel, int* status, const int* __restrict__ full) {
   using T = float;
-  using F = LineFFT<N, +1, T>;
-  using F2 = LineFFT2<N, +1>;
+  using F = LineFFTM<N, +1, T>;
+  using F2 = LineFFT2M<N, +1>;
   constexpr int W = kTileW;
   constexpr int SX = F::SMEM + ((1 - F::SMEM % 8) + 8) % 8;
   constexpr int Y = Box<N>::Y, K = Box<N>::K, XT = Box<N>::XT;
@@ -421,10 +421,10 @@ pass_a_pk(Geom3<float> g, Fields4<float> in, cpx<float>* __restrict__ out,
 // pass B: y-inverse.  grid (XT, N, NF): tile B1[f][xt][z] = [ky][W] -> B2 rows
 // ---------------------------------------------------------------------------
 template <typename T, int N>
-__global__ void __launch_bounds__(kTileW * LineFFT<N, 1, T>::G)
+__global__ void __launch_bounds__(kTileW * LineFFTM<N, 1, T>::G)
 pass_b(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
        const cpx<T>* __restrict__ tw, int* status, const int* __restrict__ full) {
-  using F = LineFFT<N, +1, T>;
+  using F = LineFFTM<N, +1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -473,8 +473,8 @@ pass_b(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
 // ---------------------------------------------------------------------------
 template <typename T, int N>
 struct RowOps {
-  using FI = LineFFT<N, +1, T>;
-  using FO = LineFFT<N, -1, T, true>;  // consumes FI's output distribution
+  using FI = LineFFTM<N, +1, T>;
+  using FO = LineFFTM<N, -1, T, true>;  // consumes FI's output distribution
   static constexpr int G = FI::G, E = FI::E;
   static constexpr int SX = RowStride<FI::SMEM, FI::G>::value;
 
@@ -523,8 +523,8 @@ struct RowOps {
       const cpx<T> z1 = line_in(A, B, r, K), z2 = line_in(C, D, r, K);
       v[e] = Pk{make_float2(z1.x, z2.x), make_float2(z1.y, z2.y)};
     }
-    if constexpr (PK == 2) LineFFT2<N, +1>::run(v, gi, tw, reinterpret_cast<float4*>(ex), WarpSync());
-    else LineFFT2<N, +1>::run(v, gi, tw, reinterpret_cast<float2*>(ex), WarpSync());
+    if constexpr (PK == 2) LineFFT2M<N, +1>::run(v, gi, tw, reinterpret_cast<float4*>(ex), WarpSync());
+    else LineFFT2M<N, +1>::run(v, gi, tw, reinterpret_cast<float2*>(ex), WarpSync());
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       ra[e] = v[e].re.x; rb[e] = v[e].im.x; rc[e] = v[e].re.y; rd[e] = v[e].im.y;
@@ -571,7 +571,7 @@ struct RowOps {
     Pk v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = Pk{make_float2(p[e], r[e]), make_float2(q[e], s ? s[e] : 0.f)};
-    using FO2 = LineFFT2<N, -1, true>;
+    using FO2 = LineFFT2M<N, -1, true>;
     if constexpr (PK == 2) FO2::run(v, gi, tw, reinterpret_cast<float4*>(ex), WarpSync());
     else FO2::run(v, gi, tw, reinterpret_cast<float2*>(ex), WarpSync());
     cpx<T> z[E];
@@ -657,8 +657,8 @@ struct RowOps {
 // before the transform, three fields out.
 constexpr int kLinAdj = 100, kLinTan = 200;
 template <typename T, int N, int NF, int L, int ST, int PK = 0>
-__global__ void __launch_bounds__(L * LineFFT<N, 1, T>::G,
-                                  (sizeof(T) == 4 && NF == 9 && L * LineFFT<N, 1, T>::G <= 128) ? 3 : 0)
+__global__ void __launch_bounds__(L * LineFFTM<N, 1, T>::G,
+                                  (sizeof(T) == 4 && NF == 9 && L * LineFFTM<N, 1, T>::G <= 128) ? 3 : 0)
 pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
        const cpx<T>* __restrict__ tw, T scale, T* __restrict__ dump, int* status, int nwt,
        unsigned long long* __restrict__ umax, int dnf) {
@@ -917,10 +917,10 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
 // pass D: y-forward.  grid (XT, N, NO): tile B3[f][xt][z] = [y][W] -> B4
 // ---------------------------------------------------------------------------
 template <typename T, int N>
-__global__ void __launch_bounds__(kTileW * LineFFT<N, 1, T>::G)
+__global__ void __launch_bounds__(kTileW * LineFFTM<N, 1, T>::G)
 pass_d(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
        const cpx<T>* __restrict__ tw, int* status, const int* __restrict__ full) {
-  using F = LineFFT<N, -1, T>;
+  using F = LineFFTM<N, -1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1204,11 +1204,11 @@ struct GroupSync {
 template <int N>
 constexpr int e_groups(int no) { return N <= 64 ? no : 2; }
 template <typename T, int N, int NO, int SCHEME>
-__global__ void __launch_bounds__(e_groups<N>(NO) * kTileW * LineFFT<N, 1, T>::G,
+__global__ void __launch_bounds__(e_groups<N>(NO) * kTileW * LineFFTM<N, 1, T>::G,
                                   N <= 64 ? 1 : sizeof(T) > 4 ? (N >= 256 ? 1 : 2) : 3)
 pass_e(Geom3<T> g, const cpx<T>* __restrict__ in, const cpx<T>* __restrict__ tw, Regs<T> R,
        StepParams<T> p, int stage, int* status, const int* __restrict__ full) {
-  using F = LineFFT<N, -1, T>;
+  using F = LineFFTM<N, -1, T>;
   constexpr int W = kTileW;
   constexpr int SX = ColStride<F::SMEM>::value;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1899,16 +1899,16 @@ struct Engine3D final : Engine3DBase {
   }
   size_t smem_e() const { return smem_e_no(nfo); }
   int col_stride() const {
-    return ColStride<LineFFT<NN, 1, T>::SMEM>::value;
+    return ColStride<LineFFTM<NN, 1, T>::SMEM>::value;
   }
   int row_stride() const {
     return RowOps<T, NN>::SX;
   }
   int fft_g() const {
-    return LineFFT<NN, 1, T>::G;
+    return LineFFTM<NN, 1, T>::G;
   }
   int fft_smem() const {
-    return LineFFT<NN, 1, T>::SMEM;
+    return LineFFTM<NN, 1, T>::SMEM;
   }
 
   int init(int n, double alpha, int scheme_) override {
@@ -1952,8 +1952,8 @@ struct Engine3D final : Engine3DBase {
     // twiddle tables: the plain plan (column passes, inverse x rows) and the
     // swapped plan (forward x rows)
     std::vector<cpx<T>> h(2 * n);
-    LineFFT<NN, 1, T>::host_table(h.data());
-    LineFFT<NN, 1, T, true>::host_table(h.data() + n);
+    LineFFTM<NN, 1, T>::host_table(h.data());
+    LineFFTM<NN, 1, T, true>::host_table(h.data() + n);
     PSG_CUDA_TRY(cudaMemcpy(tw, h.data(), sizeof(cpx<T>) * 2 * n, cudaMemcpyHostToDevice));
     PSG_CUDA_TRY(cudaMalloc(&stage_h, sizeof(double2) * (long)g.Y * g.Y * g.X));
     PSG_CUDA_TRY(cudaMalloc(&d_status, sizeof(int) * (1 + kFullSlots)));
@@ -2055,7 +2055,7 @@ struct Engine3D final : Engine3DBase {
   }
   template <int N>
   static const void* c_kernel_nf(int v, int nf) {
-    constexpr int L0 = 64 / LineFFT<N, 1, T>::G;
+    constexpr int L0 = 64 / LineFFTM<N, 1, T>::G;
     const bool pk = c_packed(v);
     const int rows = c_rows_x2(v), st = c_stages(v);
     if (rows == 1) return st == 1 ? c_fn<N, L0, 1>(nf, pk) : c_fn<N, L0, 2>(nf, pk);
@@ -2092,8 +2092,8 @@ struct Engine3D final : Engine3DBase {
   template <int N>
   int launch_c(int v, T scale, T* dp, int nf = 0, unsigned long long* um = nullptr,
                bool dep = false) {
-    constexpr int L0 = 64 / LineFFT<N, 1, T>::G;
-    constexpr int RPW = 32 / LineFFT<N, 1, T>::G;  // rows per warp tile
+    constexpr int L0 = 64 / LineFFTM<N, 1, T>::G;
+    constexpr int RPW = 32 / LineFFTM<N, 1, T>::G;  // rows per warp tile
     const int wpb = L0 * c_rows_x2(v) / RPW;       // warps per block
     const int nwt = (N * N) / RPW;
     const int nblk = (nwt + wpb - 1) / wpb;
@@ -2308,7 +2308,7 @@ struct Engine3D final : Engine3DBase {
   // pass A of the step's right-hand side, scalar or on packed transforms
   template <int N>
   int launch_a(bool chain, bool packed, Fields4<T> in, int mv, const int* full = nullptr) {
-    constexpr int G = LineFFT<N, 1, T>::G;
+    constexpr int G = LineFFTM<N, 1, T>::G;
     const int XT = g.XP / kTileW;
     const bool bous = (scheme == SCHEME_BOUS_RK4);
     if constexpr (sizeof(T) == 4) {
@@ -2332,7 +2332,7 @@ struct Engine3D final : Engine3DBase {
   // right-hand side (so that pass A may launch programmatically after it)
   template <int N>
   int rhs_n(int stage, bool want_dump, bool want_umax = false, bool chain = false) {
-    using FG = LineFFT<N, 1, T>;
+    using FG = LineFFTM<N, 1, T>;
     const int G = FG::G;
     const dim3 blk(kTileW * G);
     const int XT = g.XP / kTileW;
@@ -2522,7 +2522,7 @@ struct Engine3D final : Engine3DBase {
   // pass_a_pk's row stride, 1/k^2 table
   template <int N>
   size_t smem_a_pk_n(int ncin) const {
-    constexpr int S = LineFFT<N, 1, float>::SMEM;
+    constexpr int S = LineFFTM<N, 1, float>::SMEM;
     constexpr int SX = S + ((1 - S % 8) + 8) % 8;
     return sizeof(cpx<float>) * ((size_t)ncin * g.Y * kTileW + g.n) + 16 * (size_t)kTileW * SX +
            sizeof(float) * g.Y * kTileW;
@@ -2564,7 +2564,7 @@ struct Engine3D final : Engine3DBase {
     }
 #define PSG_SMEM(...) \
     PSG_CUDA_TRY(cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, big))
-    constexpr int L = 128 / LineFFT<N, 1, T>::G;
+    constexpr int L = 128 / LineFFTM<N, 1, T>::G;
     int nsm = 0, occ = 0;
     PSG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     if (int rc = plane_attrs<9 + kLinAdj>()) return rc;
@@ -2638,7 +2638,7 @@ struct Engine3D final : Engine3DBase {
   // products PA = F(-(E(z) x E(C x))), PB = F(-(E(C x) x E(B z))) themselves.
   template <int N, bool ADJ>
   int lin_products(Fields4<T> z, Fields4<T> x, Fields4<T> out) {
-    constexpr int G = LineFFT<N, 1, T>::G, NF = ADJ ? 9 : 12, NO = ADJ ? 6 : 3;
+    constexpr int G = LineFFTM<N, 1, T>::G, NF = ADJ ? 9 : 12, NO = ADJ ? 6 : 3;
     constexpr int L = 128 / G, RPW = 32 / G;
     const dim3 blk(kTileW * G), blk_e(e_groups<N>(NO) * kTileW * G);
     const int XT = g.XP / kTileW, nwt = N * N / RPW, nblk = nwt / (L / RPW);
@@ -2681,7 +2681,7 @@ struct Engine3D final : Engine3DBase {
   // E(i k z_rho) and E(B z_w)
   template <int N>
   int scale_products_n(Fields4<T> z, Fields4<T> x) {
-    using FG = LineFFT<N, 1, T>;
+    using FG = LineFFTM<N, 1, T>;
     const dim3 blk(kTileW * FG::G), blk2(2 * kTileW * FG::G);
     const int XT = g.XP / kTileW;
     Fields4<T> psi{};

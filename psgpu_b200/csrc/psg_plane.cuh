@@ -31,9 +31,9 @@ template <typename T, int N, int NF>
 struct Plane {
   static constexpr int CS = PlaneShape<N>::CS, NI = NF % 100;
   static constexpr int NO = NF == 9 ? 4 : NF == 9 + kLinAdj ? 6 : 3;
-  using FI = LineFFT<N, +1, T>;
-  using FO = LineFFT<N, -1, T>;
-  using FX = LineFFT<N, -1, T, true>;  // consumes FI's output distribution
+  using FI = LineFFTM<N, +1, T>;
+  using FO = LineFFTM<N, -1, T>;
+  using FX = LineFFTM<N, -1, T, true>;  // consumes FI's output distribution
   static constexpr int G = FI::G, E = FI::E, GPW = 32 / G, EXW = FI::SMEM;
   static constexpr int K = Box<N>::K, X = Box<N>::X, Y = Box<N>::Y, XT = Box<N>::XT, W = kTileW;
   static constexpr int RPC = N / CS, CPC = (X + CS - 1) / CS;  // rows, columns of a block
