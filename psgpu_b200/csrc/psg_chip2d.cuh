@@ -31,6 +31,8 @@
 // The arithmetic of the fields, products and stages is psg_ns2d.cuh's and
 // psg_tan2d.cuh's (2D_NavierStokes/src_RK4/kernels.h:82-435).
 #pragma once
+#include <type_traits>
+
 #include "psg_ns2d.cuh"
 
 namespace psg {
@@ -84,6 +86,13 @@ __device__ __forceinline__ void chip_store(cpx<float>* p, int rank, cpx<float> v
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 
+// The transforms with merged twiddles where they are the faster (us a step: 128^2
+// FP64 on 16 blocks 30 -> 25, 128^2 FP32 on one 107 -> 97, 64^2 FP64 on four 18 ->
+// 16); the tangent's registers and 256^2 at 512 threads are at their limit and
+// spill with them (128^2 FP64 tangent on 16 blocks 45 -> 55, 256^2 FP32 on eight 57
+// -> 80), and the packed forms lose too (128^2 FP32 on one block 100 -> 122).
+constexpr bool chip_merged(int n, int kind, int pk) { return n <= 128 && kind != CHIP_TANGENT && !pk; }
+
 template <typename T, int N, int CS, int KIND>
 struct ChipShape {
   using FI = LineFFT<N, +1, T>;
@@ -121,9 +130,11 @@ struct Chip2D : ChipShape<T, N, CS, KIND> {
   using S::AW; using S::BW; using S::CO; using S::CP; using S::CPC; using S::EXW; using S::G;
   using S::K; using S::NF; using S::NP; using S::NS; using S::RP; using S::RPC; using S::SW; using S::TAN;
   using S::X; using S::Y;
-  using FI = LineFFT<N, +1, T>;
-  using FO = LineFFT<N, -1, T>;
-  using FX = LineFFT<N, -1, T, true>;  // consumes FI's output distribution
+  static constexpr bool M = chip_merged(N, KIND, PK);
+  using FI = std::conditional_t<M, LineFFTM<N, +1, T>, LineFFT<N, +1, T>>;
+  using FO = std::conditional_t<M, LineFFTM<N, -1, T>, LineFFT<N, -1, T>>;
+  // consumes FI's output distribution
+  using FX = std::conditional_t<M, LineFFTM<N, -1, T, true>, LineFFT<N, -1, T, true>>;
   static constexpr int E = FI::E, GPW = 32 / G;  // points per lane, groups per warp
 
   cpx<T>*tw, *ex, *A, *B;   // twiddles, this group's exchange, rows, columns
@@ -518,5 +529,18 @@ struct Chip2D : ChipShape<T, N, CS, KIND> {
     }
   }
 };
+
+// tables of the merged transforms at grid size n: [plain plan | swapped plan], 2 n
+// entries (the others take LineFFT's)
+template <typename T>
+void chip_tables(int n, cpx<T>* h) {
+  switch (n) {
+    case 16: LineFFTM<16, 1, T>::host_table(h); LineFFTM<16, 1, T, true>::host_table(h + n); break;
+    case 32: LineFFTM<32, 1, T>::host_table(h); LineFFTM<32, 1, T, true>::host_table(h + n); break;
+    case 64: LineFFTM<64, 1, T>::host_table(h); LineFFTM<64, 1, T, true>::host_table(h + n); break;
+    case 128: LineFFTM<128, 1, T>::host_table(h); LineFFTM<128, 1, T, true>::host_table(h + n); break;
+    default: LineFFTM<256, 1, T>::host_table(h); LineFFTM<256, 1, T, true>::host_table(h + n); break;
+  }
+}
 
 }  // namespace psg

@@ -182,8 +182,8 @@ struct LineFFT {
 // difference, 2 a - (a + tau b); the first step's constant factors go the same
 // way.  Per 256-point line and lane: 340 FP instructions instead of 396; the
 // x-pass, bound by its arithmetic, went from 116 to 105 us (256^3 FP32), 229 to 184
-// (256^3 FP64) and 41 to 35 (128^3 FP64).  The 2D search's small grids and the
-// allocation-free step keep LineFFT.
+// (256^3 FP64) and 41 to 35 (128^3 FP64).  The 2D search's small grids, the
+// global-memory 2D kernels and the allocation-free step keep LineFFT.
 // ---------------------------------------------------------------------------
 
 // a, b <- a + (c + i s) b, a - (c + i s) b

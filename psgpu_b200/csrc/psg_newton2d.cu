@@ -365,7 +365,7 @@ struct Upo2D {
     const long nvec = 21 + (kmax + 1) + 10;
     const long work = 6L * n * X;
     const long per = nvec * nkt + work;
-    const long twl = 2L * n;
+    const long twl = 4L * n;  // both integrators' twiddle tables
     PSG_CUDA_TRY(cudaMalloc(&pool, sizeof(C2) * (per * ng + twl)));
     PSG_CUDA_TRY(cudaMemset(pool, 0, sizeof(C2) * (per * ng + twl)));
     G.resize(ng);
@@ -541,7 +541,8 @@ struct Upo2D {
         ci.push_back(ChipInst<T>{I.nsteps, I.mode, I.nu, I.dt, I.Z, I.D, nullptr, I.Z1});
       PSG_CUDA_TRY(cudaMemcpyAsync(plan.d_chip, ci.data(), sizeof(ChipInst<T>) * ci.size(),
                                    cudaMemcpyHostToDevice, stream));
-      PSG_CUDA_TRY(chip2d_launch<T>(cp, plan.d_chip, (int)ci.size(), plan.tw, stream));
+      PSG_CUDA_TRY(chip2d_launch<T>(cp, plan.d_chip, (int)ci.size(),
+                                    chip_merged(n, kind, 0) ? plan.tw_merged : plan.tw, stream));
       ++launches;
       if (is32)
         if (int rc = convert(out_jobs, false)) return rc;

@@ -173,12 +173,14 @@ struct Batch2D final : Batch2DBase {
       const long nk = nkt2(sizes[i]);
       sums += global[size_class(sizes[i])] ? 4 * nk + 3L * sizes[i] * (sizes[i] / 3 + 1) : nk;
     }
-    const long twlen = 2 * (16 + 32 + 64 + 128 + 256);
+    // twiddle tables of every size: the merged transforms', then LineFFT's
+    const long twlen = 2 * kTables;
     PSG_CUDA_TRY(cudaMalloc(&pool, sizeof(cpx<T>) * (total + sums + twlen)));
     PSG_CUDA_TRY(cudaMemset(pool, 0, sizeof(cpx<T>) * (total + sums + twlen)));
     twp = pool + total + sums;
     std::vector<cpx<T>> h(twlen);
-    tables2d(h.data());
+    for (int q = 0; q < kClasses; ++q) chip_tables<T>(16 << q, h.data() + (twiddles(q) - twp));
+    tables2d(h.data() + kTables);
     PSG_CUDA_TRY(cudaMemcpy(twp, h.data(), sizeof(cpx<T>) * twlen, cudaMemcpyHostToDevice));
     PSG_CUDA_TRY(cudaMalloc(&d_insts, sizeof(ChipInst<T>) * ninst));
     if (nglobal) {
@@ -257,6 +259,7 @@ struct Batch2D final : Batch2DBase {
     return true;
   }
 
+  static constexpr long kTables = 2 * (16 + 32 + 64 + 128 + 256);
   const cpx<T>* twiddles(int q) const { return twp + 2 * (16 * ((1 << q) - 1)); }
 
   // one kernel per size present, on streams of their own when there are several
@@ -283,10 +286,11 @@ struct Batch2D final : Batch2DBase {
             global_sent = true;
             PSG_CUDA_TRY(cudaMemsetAsync(d_next, 0, sizeof(int), s));
             ns2d_global<T><<<global_grid, kGlobalThreads, global_smem, s>>>(d_global, nglobal, d_next,
-                                                                          twiddles(3), twiddles(4));
+                                                                          twiddles(3) + kTables, twiddles(4) + kTables);
             PSG_CUDA_TRY(cudaGetLastError());
           }
-      } else PSG_CUDA_TRY(chip2d_launch<T>(plan_of(q, v), d_insts + off, count[q], twiddles(q), s));
+      } else PSG_CUDA_TRY(chip2d_launch<T>(plan_of(q, v), d_insts + off, count[q],
+                                           twiddles(q) + (chip_merged(16 << q, CHIP_STEP, (pk_mask >> q) & 1) ? 0 : kTables), s));
       if (present > 1) {
         PSG_CUDA_TRY(cudaEventRecord(ev_join[q], s));
         PSG_CUDA_TRY(cudaStreamWaitEvent(st, ev_join[q], 0));

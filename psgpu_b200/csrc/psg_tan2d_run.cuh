@@ -143,7 +143,8 @@ inline void tan2d_tables(int n, cpx<T>* h) {
 // dynamic shared memory and the resident-block capacity of the device
 template <typename T>
 struct IntPlan {
-  cpx<T>* tw = nullptr;
+  cpx<T>* tw = nullptr;         // LineFFT's tables, 2 n entries
+  cpx<T>* tw_merged = nullptr;  // the merged transforms', the next 2 n
   InstTan2D<T>* d_inst = nullptr;
   ChipInst<T>* d_chip = nullptr;  // the on-chip integrator's descriptors
   size_t smem = 0;
@@ -151,9 +152,11 @@ struct IntPlan {
 
   int init(int n, int ng, cpx<T>* tw_dev) {
     tw = tw_dev;
-    std::vector<cpx<T>> h(2 * n);
+    tw_merged = tw + 2 * n;
+    std::vector<cpx<T>> h(4 * n);
     tan2d_tables<T>(n, h.data());
-    PSG_CUDA_TRY(cudaMemcpy(tw, h.data(), sizeof(cpx<T>) * 2 * n, cudaMemcpyHostToDevice));
+    chip_tables<T>(n, h.data() + 2 * n);
+    PSG_CUDA_TRY(cudaMemcpy(tw, h.data(), sizeof(cpx<T>) * 4 * n, cudaMemcpyHostToDevice));
     PSG_CUDA_TRY(cudaMalloc(&d_inst, sizeof(InstTan2D<T>) * ng));
     PSG_CUDA_TRY(cudaMalloc(&d_chip, sizeof(ChipInst<T>) * ng));
     smem = tan2d_smem<T>(n);
