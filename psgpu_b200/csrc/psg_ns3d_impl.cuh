@@ -1813,10 +1813,9 @@ struct Engine3D final : Engine3DBase {
   // tangent of X0 after a tangent step, valid while lin_dx is set
   Fields4<T> LX{}, LDX{};
   bool lin_dx = false;
-  // the passes' buffers over the linearised step's fields (the engine's own for
-  // the Boussinesq scheme, whose nine fields they hold) and the x-pass's resident
-  // blocks (tangent, adjoint)
-  cpx<T>*LB1 = nullptr, *LB2 = nullptr, *lin_buf = nullptr;
+  // the passes' buffers over the linearised step's fields and the x-pass's
+  // resident blocks (tangent, adjoint)
+  cpx<T>*LB1 = nullptr, *LB2 = nullptr;
   int lin_resident[2] = {1, 1};
   Fields4<T> SA{}, SB{};       // Boussinesq adjoint products: psi (i k rho) | psi u
   int c_variant = 0;           // x-pass variant chosen by the autotuner
@@ -1980,8 +1979,7 @@ struct Engine3D final : Engine3DBase {
     if (d_rms) cudaFree(d_rms);
     d_rms = nullptr;
     if (lin) cudaFree(lin);
-    if (lin_buf) cudaFree(lin_buf);
-    lin = lin_buf = nullptr;
+    lin = nullptr;
     d_energ = nullptr; d_umax = nullptr; d_flux = nullptr;
     pool = nullptr; stage_h = nullptr; dump = nullptr; d_status = nullptr;
   }
@@ -2610,15 +2608,16 @@ struct Engine3D final : Engine3DBase {
     Fields4<T>* st[kState] = {&Zb[0], &Zb[1], &Zb[2], &Zb[3], &LA, &LN, &LS,
                               &LZ, &LK1, &LK2, &LK3, &LD, &LT, &LX, &LDX};
     const long words = ((long)kState * nc + 3 + 3 + (nc > 3 ? 6 : 0)) * box;
+    // The fields of a right-hand side take the engine's own B1 and B2 end to end
+    // (twelve fields of n Y rows fit in six of n Y and six of n n); the x-pass's
+    // input, or up to 64^3 the plane kernel's output, is a buffer of its own after
+    // the registers, in the same allocation.  The Boussinesq engine's buffers hold
+    // its nine fields as they are.
+    static_assert(12 * Box<NN>::Y <= 6 * (Box<NN>::Y + NN), "twelve fields in B1 and B2");
+    const long n2 = nc == 4 ? 0 : (NN <= 64 ? 6L * g.n * g.Y * g.XP : 12L * g.n * g.n * g.XP);
+    PSG_CUDA_TRY(cudaMalloc(&lin, sizeof(cpx<T>) * (words + n2)));
     LB1 = B1;
-    LB2 = B2;
-    if (nc == 3) {
-      const long n1 = 12L * g.n * g.Y * g.XP, n2 = 12L * g.n * g.n * g.XP;
-      PSG_CUDA_TRY(cudaMalloc(&lin_buf, sizeof(cpx<T>) * (n1 + n2)));
-      LB1 = lin_buf;
-      LB2 = lin_buf + n1;
-    }
-    PSG_CUDA_TRY(cudaMalloc(&lin, sizeof(cpx<T>) * words));
+    LB2 = nc == 4 ? B2 : lin + words;
     PSG_CUDA_TRY(cudaMemsetAsync(lin, 0, sizeof(cpx<T>) * words, stream));
     cpx<T>* p = lin;
     auto carve = [&](Fields4<T>& f, int k) {
