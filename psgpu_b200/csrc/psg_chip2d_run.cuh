@@ -37,7 +37,7 @@ struct ChipSizes {
   static constexpr bool D = sizeof(T) == 8;
   static constexpr bool built(int n, int cs, int kind) {
     return n <= 32   ? cs == 1
-           : n == 64 ? cs == 1 || cs == 4
+           : n == 64 ? cs == 1 || cs == 4 || cs == 8
            : n == 128 ? (D ? (cs == 4 && kind != CHIP_TANGENT) || cs == 8 || cs == 16
                            : (cs == 1 && kind == CHIP_STEP) || cs == 2 || cs == 4 || cs == 8)
                       : (D ? cs == 16 && kind != CHIP_TANGENT : cs == 8 || cs == 16);

@@ -465,6 +465,23 @@ struct Upo2D {
     return PSG_OK;
   }
 
+  // the launch shapes the on-chip integrator has for a kind, smallest cluster
+  // first (asked of the device once: the queries cost 0.1 ms)
+  std::vector<ChipPlan> plans_[2][3];
+  bool planned_[2][3] = {};
+  template <typename T>
+  const std::vector<ChipPlan>& chip_plans(int kind) {
+    constexpr int w = sizeof(T) == 4;
+    if (!planned_[w][kind]) {
+      ChipPlan p;
+      for (int c = 1; c <= 16; c *= 2)
+        for (int th = 128; th <= 256; th *= 2)
+          if (chip2d_plan<T>(n, c, kind, 0, th, &p)) plans_[w][kind].push_back(p);
+      planned_[w][kind] = true;
+    }
+    return plans_[w][kind];
+  }
+
   // The on-chip integrator's launch shape for `ni` integrations of `kind`: the
   // cluster size and threads with the least expected time, waves of resident
   // clusters times the time of one (a step of one 128^2 FP64 tangent: 62 us on 8
@@ -479,15 +496,13 @@ struct Upo2D {
     if (n <= 32) return false;
     static const double rel[5] = {1.0, 0.65, 0.42, 0.27, 0.21};  // 1, 2, 4, 8, 16 blocks
     double best = 0.0;
-    ChipPlan p;
-    for (int c = 0; c < 5; ++c) {
-      if ((1 << c) > cluster_max && best > 0.0) break;
-      for (int th = 128; th <= 256; th *= 2) {
-        if (!chip2d_plan<T>(n, 1 << c, kind, 0, th, &p)) continue;
-        const double waves = (ni + p.resident - 1) / p.resident;
-        const double cost = waves * rel[c] * (p.threads <= 128 ? 1.1 : 1.0);
-        if (best == 0.0 || cost < best) { best = cost; *out = p; }
-      }
+    for (const ChipPlan& p : chip_plans<T>(kind)) {
+      if (p.cs > cluster_max && best > 0.0) break;
+      int c = 0;
+      while ((1 << c) < p.cs) ++c;
+      const double waves = (ni + p.resident - 1) / p.resident;
+      const double cost = waves * rel[c] * (p.threads <= 128 ? 1.1 : 1.0);
+      if (best == 0.0 || cost < best) { best = cost; *out = p; }
     }
     return best > 0.0;
   }

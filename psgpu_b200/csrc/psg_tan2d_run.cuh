@@ -146,7 +146,7 @@ struct IntPlan {
   cpx<T>* tw = nullptr;         // LineFFT's tables, 2 n entries
   cpx<T>* tw_merged = nullptr;  // the merged transforms', the next 2 n
   InstTan2D<T>* d_inst = nullptr;
-  ChipInst<T>* d_chip = nullptr;  // the on-chip integrator's descriptors
+  ChipInst<T>* d_chip = nullptr;  // the on-chip integrator's descriptors (after d_inst)
   size_t smem = 0;
   int grid_cap = 148;
 
@@ -157,8 +157,8 @@ struct IntPlan {
     tan2d_tables<T>(n, h.data());
     chip_tables<T>(n, h.data() + 2 * n);
     PSG_CUDA_TRY(cudaMemcpy(tw, h.data(), sizeof(cpx<T>) * 4 * n, cudaMemcpyHostToDevice));
-    PSG_CUDA_TRY(cudaMalloc(&d_inst, sizeof(InstTan2D<T>) * ng));
-    PSG_CUDA_TRY(cudaMalloc(&d_chip, sizeof(ChipInst<T>) * ng));
+    PSG_CUDA_TRY(cudaMalloc(&d_inst, (sizeof(InstTan2D<T>) + sizeof(ChipInst<T>)) * ng));
+    d_chip = reinterpret_cast<ChipInst<T>*>(d_inst + ng);
     smem = tan2d_smem<T>(n);
     const void* fns[3] = {tan2d_fn<T, 1>(n), tan2d_fn<T, 2>(n), tan2d_fn<T, 4>(n)};
     for (const void* f : fns)
@@ -176,7 +176,6 @@ struct IntPlan {
   void release() {
     if (d_inst) cudaFree(d_inst);
     d_inst = nullptr;
-    if (d_chip) cudaFree(d_chip);
     d_chip = nullptr;
   }
 };
