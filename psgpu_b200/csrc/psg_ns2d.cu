@@ -27,8 +27,8 @@ constexpr int kBlock2D[3] = {128, 256, 512};
 // FP64 batches of 128^2 and 256^2: their lines in FP64 need 4 and 16 blocks'
 // shared memory, so that only 33 and 7 clusters fit the device at once, and once
 // every SM has an instance of its own the cluster barriers cost more than the L2
-// traffic: 148 instances of 128^2 202 against 239 us a step, of 256^2 940
-// against 1303 (in FP32 the chip integrator is the faster at every count).
+// traffic: 148 instances of 128^2 190 against 210 us a step, of 256^2 878
+// against 1300 (in FP32 the chip integrator is the faster at every count).
 // Instances are claimed from a counter.
 constexpr int kGlobalMin[kClasses] = {0, 0, 0, 133, 97};  // instances from which it is used (0: never)
 constexpr int kGlobalThreads = 512;
@@ -200,8 +200,9 @@ struct Batch2D final : Batch2DBase {
   // Cluster size of every size present.  A batch that leaves SMs idle spreads each
   // instance over as many blocks as there is room for, the largest grids first; a
   // batch that fills the device takes the smallest cluster that holds the grid
-  // (fewest barriers and the least traffic between blocks per step).  One 128^2
-  // FP64 run: 57 us a step on 4 blocks, 37 on 8, 30 on 16; 400 of them: see DESIGN.
+  // (fewest barriers and the least traffic between blocks per step).  128^2 FP64, us
+  // a step: one run 42 on 4 blocks, 28 on 8, 25 on 16; 33 runs 42 on 4, three
+  // waves of 28 on 8.
   int choose_plans() {
     int dev = 0, nsm = 148;
     PSG_CUDA_TRY(cudaGetDevice(&dev));
@@ -235,11 +236,13 @@ struct Batch2D final : Batch2DBase {
     for (int q = kClasses - 1; q >= 0; --q) {
       if (!count[q] || global[q]) continue;
       for (int c = 2 * cs[q]; c <= 16; c *= 2) {
-        // a cluster lies in one GPC: of 16 blocks (one per SM) 7 fit the device, of
-        // 8 15, of 4 33
-        const int room = c == 16 ? 7 * 16 : c == 8 ? 15 * 8 : c == 4 ? 33 * 4 : nsm;
-        if (blocks + (long)count[q] * (c - cs[q]) > std::min(room, nsm)) break;
         if (!chip2d_plan<T>(16 << q, c, CHIP_STEP, 0, 256, &p)) continue;
+        // a cluster lies in one GPC: of 16 blocks (one per SM) 7 fit the device, of
+        // 8 15, of 4 33; of four that share their SMs with another four (64^2) 66, still
+        // the faster (us a step of 64 runs: FP64 23 against 31 on one block each, FP32
+        // 18 against 22), unlike larger clusters sharing theirs
+        const int room = c == 16 ? 7 * 16 : c == 8 ? 15 * 8 : c == 4 ? (p.resident >= 66 ? 66 : 33) * 4 : nsm;
+        if (blocks + (long)count[q] * (c - cs[q]) > room) break;
         blocks += (long)count[q] * (c - cs[q]);
         cs[q] = c;
       }
