@@ -165,8 +165,8 @@ int psg_ns3d_linear(psg_ns3d* h, int mode, double dt, void* const* in, void* con
 
 /* ---------------------------------------------------------------- 2D */
 /* A batch of independent 2D Kolmogorov-flow instances (sizes 16..256, any
- * mix) integrated by one persistent launch: one thread block per instance,
- * largest first.  The scheme is the reference's 2D RK4 step with the final
+ * mix) integrated by one graph launch: a thread-block cluster per instance (1 to
+ * 16 blocks, by the room on the device), one kernel per size, largest first.  The scheme is the reference's 2D RK4 step with the final
  * Crank-Nicolson viscous factor and the forcing -2 at (kx,ky) = (0,+-4)
  * (2D_NavierStokes/src_RK4/kernels.h:112-435).  The single-instance drop-in
  * libpsg_ns2d.so is a batch of one. */
@@ -183,11 +183,11 @@ int psg_batch2d_download(psg_batch2d* h, int i, double* Z);
 int psg_batch2d_run(psg_batch2d* h, const double* nu, const double* dt, const int* nsteps);
 /* psg_batch2d_run in two parts: set the per-instance parameters (waits for the
  * small host-to-device copy), then launch the integration as one CUDA graph
- * (reset of the work counter + the persistent kernel), which later launches
+ * (one kernel per grid size present), which later launches
  * replay without host work; the graph is captured on first launch */
 int psg_batch2d_set_params(psg_batch2d* h, const double* nu, const double* dt, const int* nsteps);
 int psg_batch2d_launch(psg_batch2d* h);
-/* time the persistent kernel at 128, 256 and 512 threads per block on the
+/* time the kernels at up to 128, 256 and 512 threads per block on the
  * current parameters (2-step runs, states restored afterwards) and keep the
  * fastest, then (FP32) pick each grid size's transform schedule, scalar or
  * packed, the same way; variant 0/1/2, ms[3] per run (-1: does not fit) */

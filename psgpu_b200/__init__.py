@@ -330,7 +330,7 @@ class NS3D:
 
 class Batch2D:
     """Independent 2D Kolmogorov-flow instances of mixed sizes, integrated by one
-    persistent kernel launch (one thread block per instance)."""
+    graph launch (a thread-block cluster per instance)."""
 
     def __init__(self, sizes, precision: int = 32):
         L = lib()
@@ -400,7 +400,7 @@ class Batch2D:
         _check(lib().psg_batch2d_launch(self._h))
 
     def autotune(self):
-        """block size of the persistent kernel: (variant, ms per 2-step run for 128,
+        """block size of the 2D kernels: (variant, ms per 2-step run for at most 128,
         256, 512 threads)"""
         v = C.c_int()
         ms = (C.c_float * 3)()

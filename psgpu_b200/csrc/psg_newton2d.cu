@@ -485,9 +485,9 @@ struct Upo2D {
   // The on-chip integrator's launch shape for `ni` integrations of `kind`: the
   // cluster size and threads with the least expected time, waves of resident
   // clusters times the time of one (a step of one 128^2 FP64 tangent: 62 us on 8
-  // blocks, 45 on 16; of a 64^2 one 75 us on one block, 33 on 4).  False where no
+  // blocks, 45 on 16; of a 64^2 one 66 us on one block, 28 on 4, 23 on 8).  False where no
   // kernel holds the grid (256^2 FP64 tangents: the global-memory integrator), and
-  // for grids up to 32^2, where there is the least to gain (19 against 33 us a
+  // for grids up to 32^2, where there is the least to gain (15 against 33 us a
   // step) and the continuation's corrector follows its FP64 restatement to 1e-7 of
   // a residual whose rounding noise the Newton steps amplify by 1e9: those keep
   // the integrator whose rounding that agreement was established with.
