@@ -33,6 +33,7 @@
 #pragma once
 #include <type_traits>
 
+#include "psg_fft2.cuh"
 #include "psg_ns2d.cuh"
 
 namespace psg {

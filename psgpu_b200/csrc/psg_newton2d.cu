@@ -564,6 +564,10 @@ struct Upo2D {
       integrations += (long)ci.size();
       return PSG_OK;
     }
+    if (!tan2d_built<T>(n)) {
+      psg_set_error("UPO grid %d: no integrator fits this device", n);
+      return PSG_ERR_UNSUPPORTED;
+    }
     // blocks per guess: every guess starts with one; while blocks are left
     // (the resident capacity of the device at the integrator's registers), the
     // guess that would finish last moves to a cluster of two, then four.

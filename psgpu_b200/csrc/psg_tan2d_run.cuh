@@ -74,33 +74,36 @@ void cvt_launch(const CvtJob* d_jobs, int njobs, int nkt, cudaStream_t st) {
   else cvt_vec<float, double><<<grid, 256, 0, st>>>(d_jobs, nkt);
 }
 
+// The grids this integrator still runs (the on-chip one takes the others): up to
+// 32^2 and, in FP64, the tangent at 256^2.
+template <typename T>
+constexpr bool tan2d_built(int n) { return n <= 32 || (n == 256 && sizeof(T) == 8); }
+
 // kernel of one precision, grid size and cluster size (1: the persistent form)
+template <typename T, int N, int CS>
+const void* tan2d_fn_n() {
+  if constexpr (!tan2d_built<T>(N)) return nullptr;
+  else if constexpr (CS == 1) return (const void*)tan2d_persistent<T, N>;
+  else return (const void*)tan2d_cluster<T, N, CS>;
+}
 template <typename T, int CS>
 const void* tan2d_fn(int n) {
-  if (CS == 1) {
-    switch (n) {
-      case 16: return (const void*)tan2d_persistent<T, 16>;
-      case 32: return (const void*)tan2d_persistent<T, 32>;
-      case 64: return (const void*)tan2d_persistent<T, 64>;
-      case 128: return (const void*)tan2d_persistent<T, 128>;
-      default: return (const void*)tan2d_persistent<T, 256>;
-    }
-  }
   switch (n) {
-    case 16: return (const void*)tan2d_cluster<T, 16, (CS == 1 ? 2 : CS)>;
-    case 32: return (const void*)tan2d_cluster<T, 32, (CS == 1 ? 2 : CS)>;
-    case 64: return (const void*)tan2d_cluster<T, 64, (CS == 1 ? 2 : CS)>;
-    case 128: return (const void*)tan2d_cluster<T, 128, (CS == 1 ? 2 : CS)>;
-    default: return (const void*)tan2d_cluster<T, 256, (CS == 1 ? 2 : CS)>;
+    case 16: return tan2d_fn_n<T, 16, CS>();
+    case 32: return tan2d_fn_n<T, 32, CS>();
+    case 256: return tan2d_fn_n<T, 256, CS>();
   }
+  return nullptr;
 }
 
 template <typename T, int N>
 void tan2d_launch_n(int cs, int m, int grid, size_t smem, cudaStream_t st,
                     const InstTan2D<T>* d, int* next, const cpx<T>* tw) {
-  if (cs == 4) tan2d_cluster<T, N, 4><<<4 * m, 256, smem, st>>>(d, m, tw);
-  else if (cs == 2) tan2d_cluster<T, N, 2><<<2 * m, 256, smem, st>>>(d, m, tw);
-  else tan2d_persistent<T, N><<<grid, 256, smem, st>>>(d, m, next, tw);
+  if constexpr (tan2d_built<T>(N)) {
+    if (cs == 4) tan2d_cluster<T, N, 4><<<4 * m, 256, smem, st>>>(d, m, tw);
+    else if (cs == 2) tan2d_cluster<T, N, 2><<<2 * m, 256, smem, st>>>(d, m, tw);
+    else tan2d_persistent<T, N><<<grid, 256, smem, st>>>(d, m, next, tw);
+  }
 }
 
 template <typename T>
@@ -109,8 +112,6 @@ void tan2d_launch(int n, int cs, int m, int grid, size_t smem, cudaStream_t st,
   switch (n) {
     case 16: tan2d_launch_n<T, 16>(cs, m, grid, smem, st, d, next, tw); break;
     case 32: tan2d_launch_n<T, 32>(cs, m, grid, smem, st, d, next, tw); break;
-    case 64: tan2d_launch_n<T, 64>(cs, m, grid, smem, st, d, next, tw); break;
-    case 128: tan2d_launch_n<T, 128>(cs, m, grid, smem, st, d, next, tw); break;
     default: tan2d_launch_n<T, 256>(cs, m, grid, smem, st, d, next, tw); break;
   }
 }
@@ -160,6 +161,7 @@ struct IntPlan {
     PSG_CUDA_TRY(cudaMalloc(&d_inst, (sizeof(InstTan2D<T>) + sizeof(ChipInst<T>)) * ng));
     d_chip = reinterpret_cast<ChipInst<T>*>(d_inst + ng);
     smem = tan2d_smem<T>(n);
+    if (!tan2d_built<T>(n)) return PSG_OK;
     const void* fns[3] = {tan2d_fn<T, 1>(n), tan2d_fn<T, 2>(n), tan2d_fn<T, 4>(n)};
     for (const void* f : fns)
       PSG_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
