@@ -40,13 +40,18 @@ int psg_version(void);
 /* building-block check: the library's line FFT on nlines contiguous lines of n
  * complex doubles (in -> out), unnormalised, sign -1 forward / +1 inverse;
  * swap selects the transposed factorisation used after another transform */
+int psg_debug_linefft(int n, int sign, int swap, const double* in, double* out, int nlines);
+/* the same for every form of the transform that the engines run (n 16..256; swap
+ * with sign -1): form 0 plain, 1 with merged twiddles (precision 32 or 64); FP32, two
+ * lines packed: 2 plain, 3 merged, 4 merged with the one-pass exchange */
+int psg_debug_line_form(int n, int sign, int swap, int form, int precision, const double* in,
+                        double* out, int nlines);
 /* Runs one block whose bounded mbarrier wait cannot succeed (a transfer that
  * is never issued), `polls` polls long (1..2^20); *status is the status word
  * the kernel leaves: PSG_DEVICE_TIMEOUT when the wait ran out.  The engines'
  * waits end the same way (2^22 polls) and their sync calls report it. */
 #define PSG_DEVICE_TIMEOUT 0x7e01
 int psg_debug_wait_timeout(int polls, int* status);
-int psg_debug_linefft(int n, int sign, int swap, const double* in, double* out, int nlines);
 
 /* ---------------------------------------------------------------- 3D */
 typedef struct psg_ns3d psg_ns3d;

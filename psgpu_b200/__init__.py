@@ -53,6 +53,7 @@ def lib():
     L.psg_last_error.restype = C.c_char_p
     L.psg_version.restype = i
     L.psg_debug_linefft.argtypes = [i, i, i, C.POINTER(C.c_double), C.POINTER(C.c_double), i]
+    L.psg_debug_line_form.argtypes = [i, i, i, i, i, C.POINTER(C.c_double), C.POINTER(C.c_double), i]
     L.psg_ns3d_create.argtypes = [C.POINTER(vp), i, d, i, i]
     L.psg_ns3d_destroy.argtypes = [vp]
     L.psg_ns3d_destroy.restype = None

@@ -194,12 +194,16 @@ struct LineFFT2 {
   }
 };
 
-// LineFFTM (merged twiddles) for two lines at once
-__device__ __forceinline__ void pbfly(Pk& a, Pk& b, float c, float s) {
-  const float2 px = pfma(b.im, psplat(-s), pfma(b.re, psplat(c), a.re));
-  const float2 py = pfma(b.re, psplat(s), pfma(b.im, psplat(c), a.im));
-  b = Pk{pfma(a.re, psplat(2.f), make_float2(-px.x, -px.y)), pfma(a.im, psplat(2.f), make_float2(-py.x, -py.y))};
-  a = Pk{px, py};
+// LineFFTM (merged twiddles) for two lines at once: bfly and bfly_i
+__device__ __forceinline__ void pbfly(Pk& a, Pk& b, float c, float t) {
+  const float2 u = pfma(b.im, psplat(-t), b.re), w = pfma(b.re, psplat(t), b.im);
+  b = Pk{pfma(u, psplat(-c), a.re), pfma(w, psplat(-c), a.im)};
+  a = Pk{pfma(u, psplat(c), a.re), pfma(w, psplat(c), a.im)};
+}
+__device__ __forceinline__ void pbfly_i(Pk& a, Pk& b, float c, float t) {
+  const float2 u = pfma(b.im, psplat(-t), b.re), w = pfma(b.re, psplat(t), b.im);
+  b = Pk{pfma(w, psplat(c), a.re), pfma(u, psplat(-c), a.im)};
+  a = Pk{pfma(w, psplat(-c), a.re), pfma(u, psplat(c), a.im)};
 }
 
 template <int R, int LEN, int SIGN>
@@ -220,7 +224,7 @@ __device__ __forceinline__ void pdft_dit_level(Pk (&v)[R]) {
         b = SIGN < 0 ? Pk{psub(a.re, b.im), padd(a.im, b.re)} : Pk{padd(a.re, b.im), psub(a.im, b.re)};
         a = p;
       } else {
-        pbfly(a, b, Omega32<float>::c(m), (float)SIGN * Omega32<float>::s(m));
+        pbfly(a, b, Omega32<float>::c(m), (float)SIGN * Omega32<float>::t(m));
       }
     }
   }
@@ -247,7 +251,7 @@ __device__ __forceinline__ void pdft_tau_level(Pk (&v)[R], const cpx<float>* tw,
     for (int s = 0; s < R; s += LEN) {
       pbfly(v[s + j], v[s + j + half], t.x, t.y);
       if (quarter > 0)  // times SIGN i
-        pbfly(v[s + j + quarter], v[s + j + quarter + half], SIGN < 0 ? t.y : -t.y, SIGN < 0 ? -t.x : t.x);
+        pbfly_i(v[s + j + quarter], v[s + j + quarter + half], SIGN < 0 ? -t.x : t.x, t.y);
     }
   }
   if constexpr (LEN < R) pdft_tau_level<R, 2 * LEN, SIGN>(v, tw, stride);
