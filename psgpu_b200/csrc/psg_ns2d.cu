@@ -212,12 +212,14 @@ struct Batch2D final : Batch2DBase {
     ChipPlan p;
     if constexpr (sizeof(T) == 8) {
       if (nglobal) {
-        const size_t a = kGlobalThreads / LineFFT<128, 1, T>::G * LineFFT<128, 1, T>::SMEM + 2 * 128;
-        const size_t b = kGlobalThreads / LineFFT<256, 1, T>::G * LineFFT<256, 1, T>::SMEM + 2 * 256;
-        global_smem = sizeof(cpx<T>) * std::max(global[3] ? a : 0, global[4] ? b : 0);
+        const size_t a = sizeof(cpx<T>) * (kGlobalThreads / LineFFT<128, 1, T>::G * LineFFT<128, 1, T>::SMEM + 2 * 128);
+        const size_t b = sizeof(cpx<T>) * (kGlobalThreads / LineFFT<256, 1, T>::G * LineFFT<256, 1, T>::SMEM + 2 * 256);
+        global_smem = std::max(global[3] ? a : 0, global[4] ? b : 0);
         int occ = 0;
+        // the limit belongs to the kernel, not to this batch: always the larger, so
+        // that no batch lowers it under another that has yet to launch
         PSG_CUDA_TRY(cudaFuncSetAttribute(ns2d_global<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)global_smem));
+                                          (int)std::max(a, b)));
         PSG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ns2d_global<T>, kGlobalThreads,
                                                                    global_smem));
         global_grid = std::min(nglobal, nsm * std::max(occ, 1));
