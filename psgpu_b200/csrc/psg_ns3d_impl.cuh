@@ -1826,6 +1826,7 @@ struct Engine3D final : Engine3DBase {
   int c_resident[16] = {1, 1, 1, 1};  // resident blocks of each x-pass variant
   float c_ms[16] = {};                 // autotuner timings (ms per launch)
   size_t plane_smem_max = 0;   // shared memory the plane kernel may use
+  bool plane_on = true;        // PSG_PLANE=0: five passes at every size
   long launches = 0;
   // optional per-pass timing with CUDA events recorded between the passes
   bool profiling = false;
@@ -1917,6 +1918,7 @@ struct Engine3D final : Engine3DBase {
     scheme = scheme_;
     if (const char* e = getenv("PSG_PDL")) pdl = atoi(e);
     if (pdl < 0 || pdl > 2) pdl = 2;
+    if (const char* e = getenv("PSG_PLANE")) plane_on = atoi(e) != 0;
     const bool bous = (scheme == SCHEME_BOUS_RK4);
     nc = bous ? 4 : 3;
     nfi = bous ? 9 : 6;
@@ -2254,10 +2256,11 @@ struct Engine3D final : Engine3DBase {
   }
 
   // threads of the plane kernel over NF fields: its widest phase's lines, whole
-  // warps, fewer where the exchange space would not fit; 0 where it is not built
-  // or does not fit at all
+  // warps, fewer where the exchange space would not fit; 0 where it is not built,
+  // does not fit at all or is switched off
   template <int NF>
   int plane_threads() const {
+    if (!plane_on) return 0;
     if constexpr (PlaneShape<NN>::built(NF, sizeof(T))) {
       using PL = Plane<T, NN, NF>;
       int nt = std::min(kPlaneThreads, (PL::lines() * PL::G + 31) / 32 * 32);
@@ -2610,11 +2613,12 @@ struct Engine3D final : Engine3DBase {
     const long words = ((long)kState * nc + 3 + 3 + (nc > 3 ? 6 : 0)) * box;
     // The fields of a right-hand side take the engine's own B1 and B2 end to end
     // (twelve fields of n Y rows fit in six of n Y and six of n n); the x-pass's
-    // input, or up to 64^3 the plane kernel's output, is a buffer of its own after
-    // the registers, in the same allocation.  The Boussinesq engine's buffers hold
-    // its nine fields as they are.
+    // input, or the plane kernel's output where both products take that kernel, is a
+    // buffer of its own after the registers, in the same allocation.  The Boussinesq
+    // engine's buffers hold its nine fields as they are.
     static_assert(12 * Box<NN>::Y <= 6 * (Box<NN>::Y + NN), "twelve fields in B1 and B2");
-    const long n2 = nc == 4 ? 0 : (NN <= 64 ? 6L * g.n * g.Y * g.XP : 12L * g.n * g.n * g.XP);
+    const bool planes = plane_threads<9 + kLinAdj>() > 0 && plane_threads<12 + kLinTan>() > 0;
+    const long n2 = nc == 4 ? 0 : (planes ? 6L * g.n * g.Y * g.XP : 12L * g.n * g.n * g.XP);
     PSG_CUDA_TRY(cudaMalloc(&lin, sizeof(cpx<T>) * (words + n2)));
     LB1 = B1;
     LB2 = nc == 4 ? B2 : lin + words;
