@@ -1783,7 +1783,8 @@ struct Engine3D final : Engine3DBase {
   // Truncated modes of the state: an upload that brings some sets its flag,
   // d_full[slot].  Every upload takes the next of the zeroed flags, so that only
   // one in kFullSlots clears them.  fresh: no step has masked the state since the upload;
-  // exposed: the caller holds the state's device pointers and may write any mode.
+  // exposed: the state may change without a call to the engine (the caller holds its
+  // device pointers, or an upload was captured into a graph).
   static constexpr int kFullSlots = 256;
   int* d_full = nullptr;
   int slot = 0;
@@ -2244,14 +2245,20 @@ struct Engine3D final : Engine3DBase {
     return R.X0;
   }
 
+  bool capturing() const {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
+  }
   // The passes' `full` flag for a right-hand side of `stage`: null when every
   // truncated mode of the state is known to be zero.  The Euler predictor keeps
   // truncated modes, a derivative writes them, and a forced mode outside the
-  // ball enters the RK4 stages.
+  // ball enters the RK4 stages.  A captured step is replayed on states that this
+  // call knows nothing of.
   const int* full_flag(int stage) const {
     const bool forced_out = (scheme == SCHEME_NS_RK4 || scheme == SCHEME_BOUS_RK4) &&
                             prm.ampfor != (T)0 && !(prm.kf >= (T)1 && prm.kf <= (T)g.K - (T)0.5);
-    if (scheme == SCHEME_EULER_HEUN || stage == STAGE_DERIV || exposed || forced_out) return PSG_WHOLE_BOX;
+    if (scheme == SCHEME_EULER_HEUN || stage == STAGE_DERIV || exposed || forced_out || capturing())
+      return PSG_WHOLE_BOX;
     return fresh ? d_full + slot : nullptr;
   }
 
@@ -2445,6 +2452,7 @@ struct Engine3D final : Engine3DBase {
   // truncated modes
   int state_from_outside() {
     fresh = true;
+    if (capturing()) exposed = true;
     if (++slot == kFullSlots) {
       slot = 0;
       PSG_CUDA_TRY(cudaMemsetAsync(d_full, 0, sizeof(int) * kFullSlots, stream));
