@@ -28,8 +28,9 @@ constexpr int kBlock2D[3] = {128, 256, 512};
 // shared memory, so that only 33 and 7 clusters fit the device at once, and once
 // every SM has an instance of its own the cluster barriers cost more than the L2
 // traffic: 148 instances of 128^2 190 against 210 us a step, of 256^2 878
-// against 1300 (in FP32 the chip integrator is the faster at every count).
-// Instances are claimed from a counter.
+// against 1300 (in FP32 the chip integrator is the faster at every count).  Also
+// for 128^2 and 256^2 where the device has no room for a cluster that holds the grid
+// (a part of a GPU).  Instances are claimed from a counter.
 constexpr int kGlobalMin[kClasses] = {0, 0, 0, 133, 97};  // instances from which it is used (0: never)
 constexpr int kGlobalThreads = 512;
 template <typename T>
@@ -110,7 +111,9 @@ struct Batch2D final : Batch2DBase {
   // per size, block-size variant and transform schedule (scalar, packed): the
   // kernel and its launch shape; fn == nullptr where it does not fit
   ChipPlan plan[kClasses][3][2];
-  // FP64 sizes run by ns2d_global: their instances, counter, blocks and scratch
+  int cs_min[kClasses] = {0, 0, 0, 0, 0};  // fewest blocks that hold the grid (0: none)
+  int cluster_max = 16;                    // largest cluster taken (PSG_2D_CLUSTER)
+  // sizes run by ns2d_global: their instances, counter, blocks and scratch
   bool global[kClasses] = {false, false, false, false, false};
   int nglobal = 0, global_grid = 0;
   size_t global_smem = 0;
@@ -162,10 +165,7 @@ struct Batch2D final : Batch2DBase {
       maxk = std::max<long>(maxk, nkt2(n));
     }
     state_words = total;
-    for (int q = 0; q < kClasses; ++q) {
-      global[q] = sizeof(T) == 8 && kGlobalMin[q] && count[q] >= kGlobalMin[q];
-      if (global[q]) nglobal += count[q];
-    }
+    if (int rc = choose_kernels()) return rc;
     // the sums of the stage increments, for sizes whose state arrays stay outside
     // shared memory; the stage registers and rows of the global-memory kernel
     for (int i = 0; i < ninst; ++i) {
@@ -197,6 +197,25 @@ struct Batch2D final : Batch2DBase {
     return PSG_OK;
   }
 
+  // which kernel runs every size present
+  int choose_kernels() {
+    if (const char* e = getenv("PSG_2D_CLUSTER")) cluster_max = std::max(1, atoi(e));
+    ChipPlan p;
+    for (int q = 0; q < kClasses; ++q) {
+      if (!count[q]) continue;
+      for (int c = 1; c <= cluster_max && c <= 16 && !cs_min[q]; c *= 2)
+        if (chip2d_plan<T>(16 << q, c, CHIP_STEP, 0, 256, &p)) cs_min[q] = c;
+      global[q] = kGlobalMin[q] && (!cs_min[q] || (sizeof(T) == 8 && count[q] >= kGlobalMin[q]));
+      if (global[q]) {
+        nglobal += count[q];
+      } else if (!cs_min[q]) {
+        psg_set_error("2D batch: no kernel for grid %d fits this device", 16 << q);
+        return PSG_ERR_UNSUPPORTED;
+      }
+    }
+    return PSG_OK;
+  }
+
   // Cluster size of every size present.  A batch that leaves SMs idle spreads each
   // instance over as many blocks as there is room for, the largest grids first; a
   // batch that fills the device takes the smallest cluster that holds the grid
@@ -210,34 +229,27 @@ struct Batch2D final : Batch2DBase {
     int cs[kClasses] = {0, 0, 0, 0, 0};
     long blocks = nglobal;
     ChipPlan p;
-    if constexpr (sizeof(T) == 8) {
-      if (nglobal) {
-        const size_t a = sizeof(cpx<T>) * (kGlobalThreads / LineFFT<128, 1, T>::G * LineFFT<128, 1, T>::SMEM + 2 * 128);
-        const size_t b = sizeof(cpx<T>) * (kGlobalThreads / LineFFT<256, 1, T>::G * LineFFT<256, 1, T>::SMEM + 2 * 256);
-        global_smem = std::max(global[3] ? a : 0, global[4] ? b : 0);
-        int occ = 0;
-        // the limit belongs to the kernel, not to this batch: always the larger, so
-        // that no batch lowers it under another that has yet to launch
-        PSG_CUDA_TRY(cudaFuncSetAttribute(ns2d_global<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)std::max(a, b)));
-        PSG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ns2d_global<T>, kGlobalThreads,
-                                                                   global_smem));
-        global_grid = std::min(nglobal, nsm * std::max(occ, 1));
-      }
+    if (nglobal) {
+      const size_t a = sizeof(cpx<T>) * (kGlobalThreads / LineFFT<128, 1, T>::G * LineFFT<128, 1, T>::SMEM + 2 * 128);
+      const size_t b = sizeof(cpx<T>) * (kGlobalThreads / LineFFT<256, 1, T>::G * LineFFT<256, 1, T>::SMEM + 2 * 256);
+      global_smem = std::max(global[3] ? a : 0, global[4] ? b : 0);
+      int occ = 0;
+      // the limit belongs to the kernel, not to this batch: always the larger, so
+      // that no batch lowers it under another that has yet to launch
+      PSG_CUDA_TRY(cudaFuncSetAttribute(ns2d_global<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)std::max(a, b)));
+      PSG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ns2d_global<T>, kGlobalThreads,
+                                                                 global_smem));
+      global_grid = std::min(nglobal, nsm * std::max(occ, 1));
     }
     for (int q = 0; q < kClasses; ++q) {
       if (!count[q] || global[q]) continue;
-      for (int c = 1; c <= 16 && !cs[q]; c *= 2)
-        if (chip2d_plan<T>(16 << q, c, CHIP_STEP, 0, 256, &p)) cs[q] = c;
-      if (!cs[q]) {
-        psg_set_error("2D batch: no kernel for grid %d fits this device", 16 << q);
-        return PSG_ERR_UNSUPPORTED;
-      }
+      cs[q] = cs_min[q];
       blocks += (long)count[q] * cs[q];
     }
     for (int q = kClasses - 1; q >= 0; --q) {
       if (!count[q] || global[q]) continue;
-      for (int c = 2 * cs[q]; c <= 16; c *= 2) {
+      for (int c = 2 * cs[q]; c <= cluster_max && c <= 16; c *= 2) {
         if (!chip2d_plan<T>(16 << q, c, CHIP_STEP, 0, 256, &p)) continue;
         // a cluster lies in one GPC: of 16 blocks (one per SM) 7 fit the device, of
         // 8 15, of 4 33; of four that share their SMs with another four (64^2) 66, still
@@ -286,14 +298,13 @@ struct Batch2D final : Batch2DBase {
       cudaStream_t s = present > 1 ? side[q] : st;
       if (present > 1) PSG_CUDA_TRY(cudaStreamWaitEvent(s, ev_fork, 0));
       if (global[q]) {  // all such sizes in the first one's launch
-        if constexpr (sizeof(T) == 8)
-          if (!global_sent) {
-            global_sent = true;
-            PSG_CUDA_TRY(cudaMemsetAsync(d_next, 0, sizeof(int), s));
-            ns2d_global<T><<<global_grid, kGlobalThreads, global_smem, s>>>(d_global, nglobal, d_next,
-                                                                          twiddles(3) + kTables, twiddles(4) + kTables);
-            PSG_CUDA_TRY(cudaGetLastError());
-          }
+        if (!global_sent) {
+          global_sent = true;
+          PSG_CUDA_TRY(cudaMemsetAsync(d_next, 0, sizeof(int), s));
+          ns2d_global<T><<<global_grid, kGlobalThreads, global_smem, s>>>(d_global, nglobal, d_next,
+                                                                        twiddles(3) + kTables, twiddles(4) + kTables);
+          PSG_CUDA_TRY(cudaGetLastError());
+        }
       } else PSG_CUDA_TRY(chip2d_launch<T>(plan_of(q, v), d_insts + off, count[q],
                                            twiddles(q) + (chip_merged(16 << q, CHIP_STEP, (pk_mask >> q) & 1) ? 0 : kTables), s));
       if (present > 1) {

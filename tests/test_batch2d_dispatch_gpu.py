@@ -40,3 +40,20 @@ def test_two_large_fp64_batches_alive():
     assert _error(c, 0, 128) < 1e-12
     for x in (a, c, d):
         x.close()
+
+
+@pytest.mark.parametrize("prec,n,most", [(64, 256, 8), (64, 128, 2), (32, 256, 4), (64, 64, 2), (32, 64, 4), (32, 128, 2)])
+def test_no_room_for_the_cluster(monkeypatch, prec, n, most):
+    """PSG_2D_CLUSTER bounds the cluster, as a part of a GPU does: grids that need
+    more blocks run on the global-memory kernel, beside sizes that fit.  Three steps,
+    tolerance as for the on-chip kernels."""
+    monkeypatch.setenv("PSG_2D_CLUSTER", str(most))
+    sizes = [n, 32, n]
+    b = P.Batch2D(sizes, precision=prec)
+    for i, m in enumerate(sizes):
+        b.upload(i, kolmogorov_ic2d(m, 50 + m))
+    b.run(np.full(3, 0.02), 0.005, np.full(3, 3, np.int32))
+    for i, m in enumerate(sizes):
+        ref = O.ns2d_timestep(kolmogorov_ic2d(m, 50 + m), m, 0.02, 0.005, 3)[0]
+        assert np.max(np.abs(b.download(i) - ref)) < {64: 1e-12, 32: 2e-6}[prec] * np.max(np.abs(ref))
+    b.close()
