@@ -31,7 +31,10 @@ constexpr int kBlock2D[3] = {128, 256, 512};
 // against 1300 (in FP32 the chip integrator is the faster at every count).  Also
 // for 128^2 and 256^2 where the device has no room for a cluster that holds the grid
 // (a part of a GPU).  Instances are claimed from a counter.
-constexpr int kGlobalMin[kClasses] = {0, 0, 0, 133, 97};  // instances from which it is used (0: never)
+// Instances from which it is used (0: never), measured where `kGlobalRoom` of the
+// grid's smallest clusters fit the device; where more or fewer do, in proportion.
+constexpr int kGlobalMin[kClasses] = {0, 0, 0, 133, 97};
+constexpr int kGlobalRoom[kClasses] = {0, 0, 0, 33, 7};
 constexpr int kGlobalThreads = 512;
 template <typename T>
 __global__ void __launch_bounds__(kGlobalThreads)
@@ -205,7 +208,8 @@ struct Batch2D final : Batch2DBase {
       if (!count[q]) continue;
       for (int c = 1; c <= cluster_max && c <= 16 && !cs_min[q]; c *= 2)
         if (chip2d_plan<T>(16 << q, c, CHIP_STEP, 0, 256, &p)) cs_min[q] = c;
-      global[q] = kGlobalMin[q] && (!cs_min[q] || (sizeof(T) == 8 && count[q] >= kGlobalMin[q]));
+      global[q] = kGlobalMin[q] && (!cs_min[q] || (sizeof(T) == 8 && (long)count[q] * kGlobalRoom[q] >=
+                                                                         (long)kGlobalMin[q] * p.resident));
       if (global[q]) {
         nglobal += count[q];
       } else if (!cs_min[q]) {
@@ -251,11 +255,11 @@ struct Batch2D final : Batch2DBase {
       if (!count[q] || global[q]) continue;
       for (int c = 2 * cs[q]; c <= cluster_max && c <= 16; c *= 2) {
         if (!chip2d_plan<T>(16 << q, c, CHIP_STEP, 0, 256, &p)) continue;
-        // a cluster lies in one GPC: of 16 blocks (one per SM) 7 fit the device, of
-        // 8 15, of 4 33; of four that share their SMs with another four (64^2) 66, still
-        // the faster (us a step of 64 runs: FP64 23 against 31 on one block each, FP32
-        // 18 against 22), unlike larger clusters sharing theirs
-        const int room = c == 16 ? 7 * 16 : c == 8 ? 15 * 8 : c == 4 ? (p.resident >= 66 ? 66 : 33) * 4 : nsm;
+        // an SM to every block; clusters of four may share their SMs with another four
+        // (64^2), still the faster (us a step of 64 runs: FP64 23 against 31 on one block
+        // each, FP32 18 against 22), unlike larger clusters sharing theirs
+        const int alone = chip_alone(p);
+        const long room = (long)c * (c == 4 && p.resident >= 2 * alone ? 2 * alone : alone);
         if (blocks + (long)count[q] * (c - cs[q]) > room) break;
         blocks += (long)count[q] * (c - cs[q]);
         cs[q] = c;
