@@ -323,6 +323,10 @@ int psg_upo2d_set_arc(psg_upo2d* h, int i, const double* dZrdr, const double* Zr
                       double ndelta);
 int psg_upo2d_get_nu(psg_upo2d* h, int i, double* nu);
 int psg_upo2d_trace_count(psg_upo2d* h, int i);
+/* the on-chip launch shape that `count` integrations of a mode of psg_upo2d_apply take
+ * in a precision (32 or 64): blocks of a cluster and threads of a block; 0 and 0 where
+ * the global-memory integrator runs them */
+int psg_upo2d_shape(psg_upo2d* h, int mode, int precision, int count, int* blocks, int* threads);
 long psg_upo2d_integrations(psg_upo2d* h);
 long psg_upo2d_launches(psg_upo2d* h);
 /* Phase timing of psg_upo2d_solve.  psg_upo2d_profile(h, 1) clears the counters

@@ -139,6 +139,7 @@ def _declare_2d(L):
     L.psg_upo2d_integrations.restype = C.c_long
     L.psg_upo2d_trace.argtypes = [vp, i, i, dp]
     L.psg_upo2d_trace_count.argtypes = [vp, i]
+    L.psg_upo2d_shape.argtypes = [vp, i, i, i, C.POINTER(C.c_int), C.POINTER(C.c_int)]
     L.psg_upo2d_launches.argtypes = [vp]
     L.psg_upo2d_launches.restype = C.c_long
     L.psg_upo2d_set_arc.argtypes = [vp, i, dp, dp] + [C.c_double] * 7
@@ -648,6 +649,13 @@ class UPO2D:
                         "delta": rec[3], "mu": rec[4], "T": rec[5], "sx": rec[6],
                         "ner": rec[7], "normfn": rec[8], "dt": rec[9], "nu": rec[10]})
         return out
+
+    def shape(self, mode, precision=64, count=1):
+        """(blocks, threads) of the on-chip launch that `count` integrations take;
+        (0, 0): the global-memory integrator"""
+        b, t = C.c_int(), C.c_int()
+        _check(lib().psg_upo2d_shape(self._h, mode, precision, count, C.byref(b), C.byref(t)))
+        return b.value, t.value
 
     @property
     def integrations(self):

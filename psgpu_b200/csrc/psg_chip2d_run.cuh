@@ -9,10 +9,11 @@
 namespace psg {
 
 // A kernel ready to launch: cluster size, threads, shared memory, whether the
-// state arrays live in shared memory, and the clusters the device holds at once.
+// state arrays live in shared memory, and the clusters the device holds at once
+// (`alone`: with an SM to every block; filled in where it is asked for).
 struct ChipPlan {
   const void* fn = nullptr;
-  int cs = 0, threads = 0, state = 0, resident = 0;
+  int cs = 0, threads = 0, state = 0, resident = 0, alone = 0;
   size_t smem = 0;
 };
 

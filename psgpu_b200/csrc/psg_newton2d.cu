@@ -476,7 +476,10 @@ struct Upo2D {
       ChipPlan p;
       for (int c = 1; c <= 16; c *= 2)
         for (int th = 128; th <= 256; th *= 2)
-          if (chip2d_plan<T>(n, c, kind, 0, th, &p)) plans_[w][kind].push_back(p);
+          if (chip2d_plan<T>(n, c, kind, 0, th, &p)) {
+            p.alone = chip_alone(p);
+            plans_[w][kind].push_back(p);
+          }
       planned_[w][kind] = true;
     }
     return plans_[w][kind];
@@ -484,24 +487,30 @@ struct Upo2D {
 
   // The on-chip integrator's launch shape for `ni` integrations of `kind`: the
   // cluster size and threads with the least expected time, waves of resident
-  // clusters times the time of one (a step of one 128^2 FP64 tangent: 62 us on 8
-  // blocks, 45 on 16; of a 64^2 one 66 us on one block, 28 on 4, 23 on 8).  False where no
-  // kernel holds the grid (256^2 FP64 tangents: the global-memory integrator), and
-  // for grids up to 32^2, where there is the least to gain (15 against 33 us a
-  // step) and the continuation's corrector follows its FP64 restatement to 1e-7 of
-  // a residual whose rounding noise the Newton steps amplify by 1e9: those keep
-  // the integrator whose rounding that agreement was established with.
+  // clusters times the time of one, relative to the fewest blocks that hold the grid.
+  // us a step of one integration: 64^2 on 1 / 4 / 8 blocks FP64 tangent 65 / 29 / 24, base
+  // 30 / 16 / 14, FP32 tangent 44 / 22 / 18; 128^2 on 4 / 8 / 16 FP64 base 42 / 28 / 25, FP64
+  // tangent - / 59 / 44, FP32 tangent 64 / 46 / -.  Clusters that share their SMs take
+  // 1.3 to 1.4 times as long (64^2 FP64 tangent: 66 on 4 blocks 41, 33 on 8 blocks 30).
+  // False where no kernel holds the grid (256^2 FP64 tangents: the global-memory
+  // integrator), and for grids up to 32^2, which keep that integrator although it is
+  // the slower (33 against 15 us a step): a continuation's corrector is compared
+  // with its FP64 restatement at 1e-7 of a residual in which the Newton steps
+  // have amplified the last bits by 1e9, and only one order of rounding meets that.
   template <typename T>
   bool chip_shape(int kind, int ni, ChipPlan* out) {
     if (n <= 32) return false;
-    static const double rel[5] = {1.0, 0.65, 0.42, 0.27, 0.21};  // 1, 2, 4, 8, 16 blocks
+    static const double rel64[5] = {1.0, 0.65, 0.44, 0.36, 0.30};  // 1, 2, 4, 8, 16 blocks
+    static const double rel128[5] = {1.0, 0.65, 0.42, 0.29, 0.22};
+    const double* rel = n == 64 ? rel64 : rel128;
     double best = 0.0;
     for (const ChipPlan& p : chip_plans<T>(kind)) {
       if (p.cs > cluster_max && best > 0.0) break;
       int c = 0;
       while ((1 << c) < p.cs) ++c;
       const double waves = (ni + p.resident - 1) / p.resident;
-      const double cost = waves * rel[c] * (p.threads <= 128 ? 1.1 : 1.0);
+      const bool shared = std::min(ni, p.resident) > p.alone;
+      const double cost = waves * rel[c] * (p.threads <= 128 ? 1.1 : 1.0) * (shared ? 1.35 : 1.0);
       if (best == 0.0 || cost < best) { best = cost; *out = p; }
     }
     return best > 0.0;
@@ -1376,6 +1385,18 @@ extern "C" int psg_upo2d_trace_count(psg_upo2d* h, int i) {
   return (int)h->u->G[i].trace.size();
 }
 
+extern "C" int psg_upo2d_shape(psg_upo2d* h, int mode, int precision, int count, int* blocks, int* threads) {
+  if (!h || !h->u || !blocks || !threads || mode < 0 || mode > 2 || count < 1 || (precision != 32 && precision != 64)) {
+    psg_set_error("bad arguments");
+    return PSG_ERR_ARG;
+  }
+  const int kind = mode == 0 ? CHIP_TANGENT : CHIP_BASE;
+  ChipPlan p;
+  const bool chip = precision == 64 ? h->u->chip_shape<double>(kind, count, &p) : h->u->chip_shape<float>(kind, count, &p);
+  *blocks = chip ? p.cs : 0;
+  *threads = chip ? p.threads : 0;
+  return PSG_OK;
+}
 extern "C" long psg_upo2d_integrations(psg_upo2d* h) { return (h && h->u) ? h->u->integrations : -1; }
 extern "C" long psg_upo2d_launches(psg_upo2d* h) { return (h && h->u) ? h->u->launches : -1; }
 
