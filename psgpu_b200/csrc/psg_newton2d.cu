@@ -519,6 +519,12 @@ struct Upo2D {
   template <typename T>
   int integrate_t(const std::vector<IntReq>& reqs, IntPlan<T>& plan) {
     constexpr bool is32 = sizeof(T) == 4;
+    std::vector<IntReq> one, rest;
+    for (const IntReq& r : reqs) (r.mode == reqs[0].mode ? one : rest).push_back(r);
+    if (!rest.empty() && !tan2d_built<T>(n)) {  // the on-chip kernels run one kind each
+      if (int rc = integrate_t<T>(one, plan)) return rc;
+      return integrate_t<T>(rest, plan);
+    }
     std::vector<InstTan2D<T>> h;
     std::vector<CvtJob> in_jobs, out_jobs;
     for (const IntReq& r : reqs) {
@@ -552,10 +558,8 @@ struct Upo2D {
     if (is32)
       if (int rc = convert(in_jobs, true)) return rc;
     const int kind = reqs[0].mode == 0 ? CHIP_TANGENT : CHIP_BASE;
-    bool same = true;
-    for (const IntReq& r : reqs) same = same && r.mode == reqs[0].mode;
     ChipPlan cp;
-    if (same && chip_shape<T>(kind, (int)h.size(), &cp)) {
+    if (rest.empty() && chip_shape<T>(kind, (int)h.size(), &cp)) {
       // one cluster per guess, the longest integrations first
       std::stable_sort(h.begin(), h.end(), [](const InstTan2D<T>& a, const InstTan2D<T>& b) {
         return a.nsteps > b.nsteps;
