@@ -101,50 +101,14 @@ __device__ __forceinline__ void pdft(Pk (&v)[R]) {
 
 // Two lines through LineFFT<N, SIGN, float, SWAP>'s plan at once.  tw: that
 // plan's table (N entries (cos, sin) of exp(-2 pi i n1 k2 / N)); ex: SMEM
-// entries of 16 bytes (the two lines' complex values side by side).
+// entries of 8 bytes, the space of a scalar transform.
 template <int N, int SIGN, bool SWAP = false>
 struct LineFFT2 {
   using P = LineFFT<N, SIGN, float, SWAP>;
   static constexpr int R1 = P::R1, R2 = P::R2, G = P::G, E = P::E, A = P::A, B = P::B;
   static constexpr int SMEM = P::SMEM;
 
-  template <typename Sync>
-  static __device__ __forceinline__ void run(Pk (&v)[E], int g, const cpx<float>* tw, float4* ex,
-                                             Sync sync) {
-#pragma unroll
-    for (int a = 0; a < A; ++a) {
-      Pk w[R2];
-#pragma unroll
-      for (int n2 = 0; n2 < R2; ++n2) w[n2] = v[a * R2 + n2];
-      pdft<R2, SIGN>(w);
-      const int n1 = g + G * a;
-#pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2) {
-        const cpx<float> t = tw[k2 * R1 + n1];
-        const Pk x = (k2 == 0) ? w[k2] : pcmul(w[k2], t.x, SIGN > 0 ? -t.y : t.y);
-        ex[k2 * (R1 + 1) + n1] = make_float4(x.re.x, x.re.y, x.im.x, x.im.y);
-      }
-    }
-    sync();
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-      Pk w[R1];
-      const int k2 = g + G * b;
-#pragma unroll
-      for (int n1 = 0; n1 < R1; ++n1) {
-        const float4 q = ex[k2 * (R1 + 1) + n1];
-        w[n1] = Pk{make_float2(q.x, q.y), make_float2(q.z, q.w)};
-      }
-      pdft<R1, SIGN>(w);
-#pragma unroll
-      for (int k1 = 0; k1 < R1; ++k1) v[b * R1 + k1] = w[k1];
-    }
-    sync();
-  }
-
-  // The same transform with an exchange buffer of 8-byte entries (SMEM of
-  // them, the size a scalar transform uses): the real and the imaginary
-  // parts cross it one after the other.
+  // the real and the imaginary parts cross the exchange buffer one after the other
   template <typename Sync>
   static __device__ __forceinline__ void run(Pk (&v)[E], int g, const cpx<float>* tw, float2* ex,
                                              Sync sync) {
@@ -272,6 +236,7 @@ struct LineFFT2M {
   static constexpr int R1 = P::R1, R2 = P::R2, G = P::G, E = P::E, A = P::A, B = P::B;
   static constexpr int SMEM = P::SMEM;
 
+  // ex: SMEM entries of 16 bytes, the two lines' complex values side by side
   template <typename Sync>
   static __device__ __forceinline__ void run(Pk (&v)[E], int g, const cpx<float>* tw, float4* ex, Sync sync) {
 #pragma unroll

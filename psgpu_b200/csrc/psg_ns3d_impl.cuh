@@ -73,7 +73,7 @@ __device__ __forceinline__ int ball_reach(int s) {
 // tile's lowest kx.  Outside them every mode of the stage state is zero, and
 // every mode the passes produce is masked away: pass A transforms no such tile
 // and loads no such rows, pass B reads no such rows, pass D stores none, pass E
-// updates none of them (256^3: 17% of the tiles of A and E, 45% of the state's
+// updates none of them (256^3: 21% of the tiles of A and E, 47% of the state's
 // modes).  `full` (a device flag, null or PSG_WHOLE_BOX) lifts this: a state that
 // still holds truncated modes, as an uploaded one may, takes part with all of
 // its box.
@@ -126,20 +126,7 @@ __device__ __forceinline__ void pdl_trigger() {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Load `n` contiguous chunks into shared memory with one mbarrier; returns
-// false (uniformly) if the copy did not complete within the wait bound.
-__device__ __forceinline__ bool tile_load(uint64_t* bar, int* s_ok, void* const* dst,
-                                          const void* const* src, const uint32_t* bytes, int n,
-                                          int* status) {
-  if (threadIdx.x == 0) {
-    uint32_t tot = 0;
-    for (int i = 0; i < n; ++i) tot += bytes[i];
-    mbar_expect_tx(bar, tot);
-    for (int i = 0; i < n; ++i) bulk_g2s(dst[i], src[i], bytes[i], bar);
-  }
-  return true;
-}
-
+// false (uniformly) if the tile copy did not complete within the wait bound
 __device__ __forceinline__ bool tile_wait(uint64_t* bar, int* s_ok, int* status) {
   if (threadIdx.x == 0) *s_ok = mbar_wait_bounded(bar, 0, status) ? 1 : 0;
   __syncthreads();
@@ -507,15 +494,13 @@ struct RowOps {
   }
 
   // FP32: four real fields as two complex lines (a + i b, c + i d) through one
-  // packed f32x2 transform, the instruction count of one scalar line.  PK 1:
-  // the exchange crosses the scalar-sized buffer in two halves; PK 2: one
-  // pass through a buffer of twice the size.
-  template <int PK>
+  // packed f32x2 transform, the instruction count of one scalar line; the
+  // exchange crosses the scalar-sized buffer in two halves
   static __device__ __forceinline__ void c2r_quad(const cpx<T>* A, const cpx<T>* B, const cpx<T>* C,
                                                   const cpx<T>* D, int K, int gi, const cpx<T>* tw,
                                                   cpx<T>* ex, T (&ra)[E], T (&rb)[E], T (&rc)[E],
                                                   T (&rd)[E]) {
-    static_assert(sizeof(T) == 4 && PK >= 1 && PK <= 2, "packed transforms are FP32");
+    static_assert(sizeof(T) == 4, "packed transforms are FP32");
     Pk v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -523,8 +508,7 @@ struct RowOps {
       const cpx<T> z1 = line_in(A, B, r, K), z2 = line_in(C, D, r, K);
       v[e] = Pk{make_float2(z1.x, z2.x), make_float2(z1.y, z2.y)};
     }
-    if constexpr (PK == 2) LineFFT2M<N, +1>::run(v, gi, tw, reinterpret_cast<float4*>(ex), WarpSync());
-    else LineFFT2M<N, +1>::run(v, gi, tw, reinterpret_cast<float2*>(ex), WarpSync());
+    LineFFT2M<N, +1>::run(v, gi, tw, reinterpret_cast<float2*>(ex), WarpSync());
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       ra[e] = v[e].re.x; rb[e] = v[e].im.x; rc[e] = v[e].re.y; rd[e] = v[e].im.y;
@@ -560,20 +544,18 @@ struct RowOps {
   // FP32: forward transforms of (p + i q) and (r + i s) as one packed line pair;
   // p, q (and r, s with s) pre-scaled by 1/2 for the split; s == nullptr: r
   // alone, stored directly into Rr
-  template <int PK>
   static __device__ __forceinline__ void r2c_quad(const T (&p)[E], const T (&q)[E], const T (&r)[E],
                                                   const T* s, int K, int XP, int gi,
                                                   const cpx<T>* tw, cpx<T>* ex,
                                                   cpx<T>* __restrict__ P, cpx<T>* __restrict__ Q,
                                                   cpx<T>* __restrict__ Rr, cpx<T>* __restrict__ S,
                                                   long tstride) {
-    static_assert(sizeof(T) == 4 && PK >= 1 && PK <= 2, "packed transforms are FP32");
+    static_assert(sizeof(T) == 4, "packed transforms are FP32");
     Pk v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = Pk{make_float2(p[e], r[e]), make_float2(q[e], s ? s[e] : 0.f)};
     using FO2 = LineFFT2M<N, -1, true>;
-    if constexpr (PK == 2) FO2::run(v, gi, tw, reinterpret_cast<float4*>(ex), WarpSync());
-    else FO2::run(v, gi, tw, reinterpret_cast<float2*>(ex), WarpSync());
+    FO2::run(v, gi, tw, reinterpret_cast<float2*>(ex), WarpSync());
     cpx<T> z[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) z[e] = cpx<T>{v[e].re.x, v[e].im.x};
@@ -647,10 +629,8 @@ struct RowOps {
 // memory), leaves the block count to the compiler (0).  Passes A and E in
 // FP64 at 256^3 likewise ask for one block per SM: their shared memory allows
 // no more, and the register cap of three would only make them spill.
-// PK (FP32 only): 0 one scalar transform per complex line; 1 or 2 two lines per
-// packed f32x2 transform (RowOps::c2r_quad / r2c_quad), with the exchange in
-// two halves through the scalar-sized buffer (1) or in one pass through a
-// buffer twice that size (2).
+// PK (FP32 only): 0 one scalar transform per complex line; 1 two lines per
+// packed f32x2 transform (RowOps::c2r_quad / r2c_quad).
 // NF 9 + kLinAdj and 12 + kLinTan: the linearised step's fields (pass A, modes 3
 // and 4) and their cross products: adjoint -(z x Cx) and -(Cx x Bz), six fields
 // out, the transforms of C x shared by both; tangent -(Bx x z) - (Bz x x), summed
@@ -701,7 +681,7 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
   if (lane == 0 && t < nwt) issue(t, 0);
   const long tstride = (long)N * N * kTileW;  // B3: successive xt tiles
   const long fstride = (long)XT * tstride;
-  cpx<T>* ex = s_ex + (warp * RPW + j) * R::SX * (PK == 2 ? 2 : 1);
+  cpx<T>* ex = s_ex + (warp * RPW + j) * R::SX;
   for (int i = 0; t < nwt; ++i, t += wstride) {
     const int b = (ST == 2) ? (i & 1) : 0;
     const uint32_t parity = (ST == 2) ? ((i >> 1) & 1) : (i & 1);
@@ -801,11 +781,11 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
       // physical fields are live); (xi + i eta, zeta + i u) -> (v + i w) else
       if constexpr (BOUS) {
         T rx[E], ry[E], n4[E];
-        R::template c2r_quad<PK>(src + 3 * fs, src + 6 * fs, src + 4 * fs, src + 7 * fs, K, gi,
+        R::c2r_quad(src + 3 * fs, src + 6 * fs, src + 4 * fs, src + 7 * fs, K, gi,
                                  s_tw, ex, u, rx, v, ry);
 #pragma unroll
         for (int e = 0; e < E; ++e) n4[e] = u[e] * rx[e] + v[e] * ry[e];
-        R::template c2r_quad<PK>(src + 5 * fs, src + 8 * fs, src, src + fs, K, gi, s_tw, ex, w, rx,
+        R::c2r_quad(src + 5 * fs, src + 8 * fs, src, src + fs, K, gi, s_tw, ex, w, rx,
                                  xi, et);
 #pragma unroll
         for (int e = 0; e < E; ++e) n4[e] = (n4[e] + w[e] * rx[e]) * hscale;
@@ -841,12 +821,12 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
           n2[e] = -(w[e] * xi[e] - u[e] * zt[e]) * hscale;
           n3[e] = -(u[e] * et[e] - v[e] * xi[e]) * hscale;
         }
-        R::template r2c_quad<PK>(n1, n2, n3, n4, K, XP, gi, two, ex, dst, dst + fstride,
+        R::r2c_quad(n1, n2, n3, n4, K, XP, gi, two, ex, dst, dst + fstride,
                                  dst + 2 * fstride, dst + 3 * fstride, tstride);
         __syncwarp();
         continue;
       }
-      R::template c2r_quad<PK>(src, src + fs, src + 2 * fs, src + 3 * fs, K, gi, s_tw, ex, xi, et,
+      R::c2r_quad(src, src + fs, src + 2 * fs, src + 3 * fs, K, gi, s_tw, ex, xi, et,
                                zt, u);
     } else {
       R::c2r_pair(src, src + fs, K, gi, s_tw, ex, xi, et);
@@ -888,7 +868,7 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
       n3[e] = -(u[e] * et[e] - v[e] * xi[e]) * (BOUS ? hscale : scale);
     }
     if constexpr (PK != 0 && !BOUS) {
-      R::template r2c_quad<PK>(n1, n2, n3, nullptr, K, XP, gi, two, ex, dst, dst + fstride,
+      R::r2c_quad(n1, n2, n3, nullptr, K, XP, gi, two, ex, dst, dst + fstride,
                                dst + 2 * fstride, nullptr, tstride);
     } else if (!BOUS) {
       R::r2c_pair(n1, n2, K, XP, gi, two, ex, dst, dst + fstride, tstride);
@@ -1188,14 +1168,6 @@ __device__ __forceinline__ void scheme_point(const Geom3<T>& g, const Regs<T>& R
   }
 
 }
-
-// barrier of the first `count` threads of the block only (hardware barrier 1)
-struct GroupSync {
-  int count;
-  __device__ __forceinline__ void operator()() const {
-    asm volatile("bar.sync 1, %0;" ::"r"(count) : "memory");
-  }
-};
 
 // Pass E runs 2 W G threads: for three fields both halves transform the tile,
 // for more the first half alone (named barriers of their own), then all of
@@ -1539,9 +1511,11 @@ __global__ void copy_fields(Fields4<T> src, Fields4<T> dst, int nc, long len) {
 // the real inner product of the stored coefficients E^T = 2 N^3 F and
 // F^T = E / (2 N^3), B and C are self-adjoint, and a.(b x c) = b.(c x a), so
 //   N'(w)^T l = B F(E(w) x E(C l)) + F(E(C l) x E(B w)).
-// Every term is one bilinear product P(a, b) = F(-(E(a) x E(b))) of the five
-// passes (pass A in pair mode, pass E in raw mode); the kernels below combine
-// the products and apply the stage arithmetic of scheme_point's RK4 branch.
+// One run of the passes forms a right-hand side: pass A the nine or twelve fields
+// (modes 3 and 4), the x-pass or the plane kernel both cross products, pass E
+// (SCHEME_LIN) their combination; for the Boussinesq adjoint pass E writes the
+// products themselves (SCHEME_RAW).  The kernels below apply the stage arithmetic of
+// scheme_point's RK4 branch.
 // ---------------------------------------------------------------------------
 template <typename T>
 struct TileMode {
@@ -1907,9 +1881,6 @@ struct Engine3D final : Engine3DBase {
   }
   int fft_g() const {
     return LineFFTM<NN, 1, T>::G;
-  }
-  int fft_smem() const {
-    return LineFFTM<NN, 1, T>::SMEM;
   }
 
   int init(int n, double alpha, int scheme_) override {
