@@ -20,8 +20,9 @@ scheme, 3D_Boussinesq/src/kernels.h:331-621, at Ri = 0).  Data are synthetic
 * ``cpu_baseline``: the FP64 CPU oracle (C + OpenMP on all host threads) on a
   bounded sample of the same workload (one RK4 step of the same scheme).
 * ``roofline``: the dominant pass (largest share of the step's device time),
-  its algorithmic HBM bytes per launch over its average CUDA-event duration,
-  against the measured copy bandwidth in MEASURED_PEAKS.json.
+  its algorithmic HBM bytes per launch (within the ball of kept modes) over its
+  average CUDA-event duration, against the measured copy bandwidth in
+  MEASURED_PEAKS.json.
 * ``fp64_engine``: device steps/s of the same workload on the FP64 engine (the
   reference's precision), Navier-Stokes RK4/CN and Boussinesq at Ri = 0.
 
@@ -123,15 +124,39 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
-def algorithmic_bytes(n, word=8, nc=3, nfi=6):
+def ball_lines(n, w=8):
+    """(kx, ky) lines and modes of the box that the passes take when they keep to the
+    ball of kept modes, in tiles of w kx columns whose reach is that of their lowest kx."""
+    K = n // 3
+    lines = modes = 0
+    for kx in range(K + 1):
+        k0 = kx // w * w
+        for ky in range(-K, K + 1):
+            q = K * K - K - k0 * k0 - ky * ky
+            if q >= 0:
+                lines += 1
+                modes += 2 * math.isqrt(q) + 1
+    return lines, modes
+
+
+def algorithmic_bytes(n, word=8, nc=3, nfi=6, ball=False):
     """HBM bytes of one right-hand side per pass, complex words of `word` bytes,
-    counting only kept modes (IKTX = n/3+1 columns, IKTY = IKTZ = 2(n/3)+1 rows)
+    counting the truncated box (IKTX = n/3+1 columns, IKTY = IKTZ = 2(n/3)+1 rows)
     and one read plus one write per pass; pass A also reads the nc stage-state
     components, pass E writes/reads the scheme registers (counted per stage in
     stage_bytes).  nc state components, nfi fields through the x-pass (3, 6
-    for Navier-Stokes; 4, 9 for Boussinesq)."""
+    for Navier-Stokes; 4, 9 for Boussinesq).  ball: only the lines and modes within
+    the ball of kept modes, which is what the passes move once a step has masked
+    the state."""
     K = n // 3
     X, Y = K + 1, 2 * K + 1
+    if ball:
+        lines, modes = ball_lines(n)
+        a = (nc * modes + nfi * lines * n) * word
+        b = (nfi * lines * n + nfi * X * n * n) * word
+        c = (nfi * X * n * n + nc * X * n * n) * word
+        d = (nc * X * n * n + nc * lines * n) * word
+        return [a, b, c, d, nc * lines * n * word]
     a = (nc * X * Y * Y + nfi * X * Y * n) * word
     b = (nfi * X * Y * n + nfi * X * n * n) * word
     c = (nfi * X * n * n + nc * X * n * n) * word
@@ -140,13 +165,13 @@ def algorithmic_bytes(n, word=8, nc=3, nfi=6):
     return [a, b, c, d, e]
 
 
-def stage_bytes(n, stage, word=8, nc=3, carried=True):
+def stage_bytes(n, stage, word=8, nc=3, carried=True, ball=False):
     """state/register traffic of pass E for RK4 stage 0..3 (nc components each):
     stages 0-2 read S and write K_s and X0; the final stage reads S, K1, K2, K3
     (and the carried rounding error of the FP32 state) and writes S, X0 (and
     that error)."""
     K = n // 3
-    nkt = (K + 1) * (2 * K + 1) ** 2
+    nkt = ball_lines(n)[1] if ball else (K + 1) * (2 * K + 1) ** 2
     arrays = 3 if stage < 3 else (8 if carried else 6)
     return arrays * nc * nkt * word
 
@@ -201,8 +226,8 @@ def run_ours(args, rank, world, dist):
 
     # roofline of the dominant pass
     peak, peak_kind = measured_peaks()
-    alg = algorithmic_bytes(N, 8)
-    per_step_stage = sum(stage_bytes(N, s) for s in range(4)) / 4.0
+    alg = algorithmic_bytes(N, 8, ball=True)
+    per_step_stage = sum(stage_bytes(N, s, ball=True) for s in range(4)) / 4.0
     shares = {}
     tot = sum(v[0] for v in prof.values())
     roof = None
@@ -226,7 +251,7 @@ def run_ours(args, rank, world, dist):
             "timed_by": "CUDA events on the engine's stream between the passes, over a segment of "
                         "min(steps, 20) steps after the headline's timed region",
             "pass_share": shares}
-    step_bytes = 4 * sum(alg) + sum(stage_bytes(N, s) for s in range(4))
+    step_bytes = 4 * sum(alg) + sum(stage_bytes(N, s, ball=True) for s in range(4))
     whole = {"algorithmic_bytes_per_step": int(step_bytes),
              "achieved_GBps": round(step_bytes / (ms / args.steps / 1e3) / 1e9, 1)}
     whole["frac"] = round(whole["achieved_GBps"] / peak, 4)
@@ -313,8 +338,8 @@ def pass_table(args, nsteps=10):
         eng.profile(False)
         nc, nfi = (4, 9) if bous else (3, 6)
         word = 8 if prec == 32 else 16
-        alg = algorithmic_bytes(n, word, nc, nfi)
-        stage = sum(stage_bytes(n, s, word, nc, carried=(prec == 32)) for s in range(4)) / 4.0
+        alg = algorithmic_bytes(n, word, nc, nfi, ball=True)
+        stage = sum(stage_bytes(n, s, word, nc, carried=(prec == 32), ball=True) for s in range(4)) / 4.0
         rows = {}
         for i, (pname, (ms, cnt)) in enumerate(prof.items()):
             b = alg[i] + (stage if i == 4 else 0)
@@ -323,7 +348,7 @@ def pass_table(args, nsteps=10):
                            "achieved_GBps": round(b / t / 1e9, 1),
                            "frac": round(b / t / 1e9 / peak, 4)}
         tot_ms = sum(v[0] for v in prof.values())
-        step_b = 4 * sum(alg) + sum(stage_bytes(n, s, word, nc, carried=(prec == 32))
+        step_b = 4 * sum(alg) + sum(stage_bytes(n, s, word, nc, carried=(prec == 32), ball=True)
                                     for s in range(4))
         out["engines"][name] = {"passes": rows, "xpass_variant": eng.autotune(rerun=False),
                                 "ms_per_step_passes": round(tot_ms / nsteps, 4),
@@ -419,7 +444,7 @@ UPO_N, UPO_NU, UPO_DT, UPO_GUESSES, UPO_KMAX = 128, 1.0 / 40.0, 0.005, 64, 60
 def upo_guesses(G=UPO_GUESSES, search=400.0, seed=5000):
     """64 guesses from turbulent 2D Kolmogorov states, Re = 40, 128^2: 64 seeded
     runs (modes 1 <= |k| <= 8, enstrophy 1) spun up for 500 time units in one
-    persistent FP32 launch, then continued for `search` time units under the
+    FP32 launch, then continued for `search` time units under the
     GPU recurrence search (every 0.1 time units, a ring of 20 time units,
     32 x 4 trial shifts over the 2 x 8^2 lowest modes, threshold 0.4).  Of the
     emitted guesses those with periods in [5, 20] are kept, lowest residual
@@ -615,8 +640,8 @@ def run_ns2d_single(args):
 
 # ------------------------------------------------------------ 2D ensemble
 def run_ensemble2d(args, rank=0, world=1, dist=None, dev=None):
-    """512 independent 2D Kolmogorov runs in one persistent launch replayed as a
-    CUDA graph: sizes uniform over {64^2, 128^2, 256^2}, Re uniform in [20, 100],
+    """512 independent 2D Kolmogorov runs in one launch, a CUDA graph with a
+    kernel per size: sizes uniform over {64^2, 128^2, 256^2}, Re uniform in [20, 100],
     forcing wavenumber 4, seeded initial vorticity (modes 1 <= |k| <= 8, phases
     uniform, amplitude ~ 1/|k|, enstrophy 1), dt = 0.005, 1000 steps each, FP32;
     block size picked by the autotuner.  Instance-steps per second on the device
@@ -677,7 +702,7 @@ def run_ensemble2d(args, rank=0, world=1, dist=None, dev=None):
     if rank != 0:
         return None
     out = {"workload": "512 x 2D Kolmogorov, sizes U{64,128,256}^2, Re U[20,100], kf=4, "
-                       "dt=0.005, 1000 steps, FP32, one persistent launch (CUDA graph) per GPU",
+                       "dt=0.005, 1000 steps, FP32, one graph launch (a kernel per size) per GPU",
            "instance_steps_per_s": round(M * steps / dev_s, 1), "seconds": round(dev_s, 4),
            "e2e_instance_steps_per_s": round(M * steps / e2e_s, 1), "e2e_seconds": round(e2e_s, 3),
            "scaling": "strong", "ranks": world, "gpu_launches": launches, "finite": bool(finite),

@@ -56,7 +56,7 @@ int psg_debug_wait_timeout(int polls, int* status);
 /* ---------------------------------------------------------------- 3D */
 typedef struct psg_ns3d psg_ns3d;
 
-/* n: grid points per direction (16..512, power of two); alpha must be 1;
+/* n: grid points per direction (16..256, power of two); alpha must be 1;
  * precision: 32 (FP32 storage and transforms) or 64. */
 int psg_ns3d_create(psg_ns3d** h, int n, double alpha, int scheme, int precision);
 void psg_ns3d_destroy(psg_ns3d* h);
@@ -106,11 +106,18 @@ int psg_ns3d_rms_accumulate(psg_ns3d* h, double count);
 int psg_ns3d_rms_download(psg_ns3d* h, double* const* out);
 int psg_ns3d_sync(psg_ns3d* h);
 long psg_ns3d_launches(psg_ns3d* h);
-/* device state pointers and padded row length (complex words) */
+/* device state pointers and padded row length (complex words).  With the pointers
+ * handed out (comps not null) the caller may write any mode of the state at any time,
+ * so from then on the engine's passes take the whole box instead of the ball of kept
+ * modes (some 15% more per step at 256^3).  A step captured into a CUDA graph does so
+ * too, and an engine one of whose uploads was captured, from then on. */
 int psg_ns3d_layout(psg_ns3d* h, int* xp, void** comps);
 /* per-pass timing: enable(1) resets and records CUDA events between the five
  * passes of every right-hand side; read returns total ms and launch counts of
- * passes A..E (z-inverse, y-inverse, x, y-forward, z-forward + update) */
+ * passes A..E (z-inverse, y-inverse, x, y-forward, z-forward + update).  While it is
+ * on, grids up to 64^3 run the five passes too, where a plain step runs passes B, C
+ * and D as one kernel (FP32 Navier-Stokes at 64^3 excepted; PSG_PLANE=0 at set-up
+ * keeps the five passes for good). */
 int psg_ns3d_profile(psg_ns3d* h, int enable);
 int psg_ns3d_profile_read(psg_ns3d* h, double* ms, long* counts);
 /* re-run the set-up autotuner (x-pass rows per block, buffers per warp and, in FP32,
@@ -171,9 +178,11 @@ int psg_ns3d_linear(psg_ns3d* h, int mode, double dt, void* const* in, void* con
 /* ---------------------------------------------------------------- 2D */
 /* A batch of independent 2D Kolmogorov-flow instances (sizes 16..256, any
  * mix) integrated by one graph launch: a thread-block cluster per instance (1 to
- * 16 blocks, by the room on the device), one kernel per size, largest first.  The scheme is the reference's 2D RK4 step with the final
- * Crank-Nicolson viscous factor and the forcing -2 at (kx,ky) = (0,+-4)
- * (2D_NavierStokes/src_RK4/kernels.h:112-435).  The single-instance drop-in
+ * 16 blocks, by the room on the device; PSG_2D_CLUSTER bounds them), one kernel per
+ * size, largest first; large FP64 batches of 128^2 and 256^2, and these grids where no
+ * cluster has room, take one block per instance with its rows in global memory.  The
+ * scheme is the reference's 2D RK4 step with the final Crank-Nicolson viscous factor
+ * and the forcing -2 at (kx,ky) = (0,+-4) (2D_NavierStokes/src_RK4/kernels.h:112-435).  The single-instance drop-in
  * libpsg_ns2d.so is a batch of one. */
 typedef struct psg_batch2d psg_batch2d;
 
@@ -184,7 +193,7 @@ int psg_batch2d_set_stream(psg_batch2d* h, void* cuda_stream);
 int psg_batch2d_upload(psg_batch2d* h, int i, const double* Z);
 int psg_batch2d_download(psg_batch2d* h, int i, double* Z);
 /* enqueue nsteps[i] steps of length dt[i] with viscosity nu[i] for every
- * instance, in one kernel launch on the handle's stream */
+ * instance, in one graph launch on the handle's stream */
 int psg_batch2d_run(psg_batch2d* h, const double* nu, const double* dt, const int* nsteps);
 /* psg_batch2d_run in two parts: set the per-instance parameters (waits for the
  * small host-to-device copy), then launch the integration as one CUDA graph

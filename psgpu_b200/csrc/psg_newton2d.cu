@@ -9,8 +9,9 @@
 // bisection on mu and the halve/double logic of the reference.  Differences in
 // form, not in algorithm:
 //   * all guesses advance in lock step and every integration of a phase (one
-//     per GMRES iteration, one per hookstep trial) is a single persistent
-//     launch over the guesses;
+//     per GMRES iteration, one per hookstep trial) is a single launch over the
+//     guesses, each on a thread-block cluster (psg_chip2d.cuh; up to 32^2, and
+//     FP64 tangents at 256^2, psg_tan2d.cuh's kernels);
 //   * Jv is the exact tangent of the discrete step (integrated with the base,
 //     psg_tan2d.cuh) in FP64 or in FP32, or the reference's forward
 //     difference (eps = 1e-7, FP64: a difference quotient of FP32
