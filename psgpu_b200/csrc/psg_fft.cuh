@@ -205,7 +205,7 @@ struct LineFFT {
 // FP32 (16 to 256 points), 0.75 to 0.90 in FP64.  (The difference as 2 a - (a +
 // tau b), six multiply-adds as well, inherits the sum's rounding: 1.07 to 1.12 and
 // 0.98 to 1.18.)  Per 256-point line and lane: 340 FP instructions instead of 396; the
-// x-pass, bound by its arithmetic, went from 116 to 105 us (256^3 FP32), 229 to 184
+// x-pass, bound by its arithmetic, went from 116 to 108 us (256^3 FP32), 229 to 188
 // (256^3 FP64) and 41 to 35 (128^3 FP64).  The 2D search's small grids, the
 // global-memory 2D kernels and the allocation-free step keep LineFFT.
 // ---------------------------------------------------------------------------
