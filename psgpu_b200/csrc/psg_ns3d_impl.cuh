@@ -896,8 +896,16 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
 // ---------------------------------------------------------------------------
 // pass D: y-forward.  grid (XT, N, NO): tile B3[f][xt][z] = [y][W] -> B4
 // ---------------------------------------------------------------------------
+// At 64^3 FP32 the pass is held to 32 registers, 32 blocks per SM: with 40, which it
+// would take, a step of passes chained by programmatic launches took 95 us instead of
+// 86 (112 as ordinary launches either way).  At 128^3 and 256^3 a cap costs the pass 6
+// to 20%.
+constexpr int d_min_blocks(int n, int elem, int threads) {
+  return n == 64 && elem == 4 ? 65536 / (threads * 32) : 0;
+}
 template <typename T, int N>
-__global__ void __launch_bounds__(kTileW * LineFFTM<N, 1, T>::G)
+__global__ void __launch_bounds__(kTileW * LineFFTM<N, 1, T>::G,
+                                  d_min_blocks(N, sizeof(T), kTileW * LineFFTM<N, 1, T>::G))
 pass_d(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
        const cpx<T>* __restrict__ tw, int* status, const int* __restrict__ full) {
   using F = LineFFTM<N, -1, T>;
