@@ -87,12 +87,15 @@ __device__ __forceinline__ void chip_store(cpx<float>* p, int rank, cpx<float> v
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 
-// The transforms with merged twiddles where they are the faster (us a step: 128^2
-// FP64 on 16 blocks 30 -> 25, 128^2 FP32 on one 107 -> 97, 64^2 FP64 on four 18 ->
-// 16); the tangent's registers and 256^2 at 512 threads are at their limit and
-// spill with them (128^2 FP64 tangent on 16 blocks 45 -> 55, 256^2 FP32 on eight 57
-// -> 80), and the packed forms lose too (128^2 FP32 on one block 100 -> 122).
-constexpr bool chip_merged(int n, int kind, int pk) { return n <= 128 && kind != CHIP_TANGENT && !pk; }
+// The transforms with merged twiddles in FP64 up to 128^2, where they are the faster
+// (us a step: 128^2 on 16 blocks 30 -> 25, 64^2 on four 18 -> 16); the tangent's
+// registers are at their limit and spill with them (128^2 tangent on 16 blocks 45 ->
+// 55).  Not in FP32, although 128^2 on one block takes 107 instead of 97: a path
+// through their tables has several rounded factors where LineFFT's has one, the same
+// error at every right-hand side, and after 20 steps the FP32 state was 1.23 (16^2 and
+// 64^2) and 1.04 (128^2) times as far from 80-bit arithmetic as with LineFFT (FP64: 0.79
+// to 0.99).
+constexpr bool chip_merged(int elem, int n, int kind) { return elem == 8 && n <= 128 && kind != CHIP_TANGENT; }
 
 template <typename T, int N, int CS, int KIND>
 struct ChipShape {
@@ -131,7 +134,7 @@ struct Chip2D : ChipShape<T, N, CS, KIND> {
   using S::AW; using S::BW; using S::CO; using S::CP; using S::CPC; using S::EXW; using S::G;
   using S::K; using S::NF; using S::NP; using S::NS; using S::RP; using S::RPC; using S::SW; using S::TAN;
   using S::X; using S::Y;
-  static constexpr bool M = chip_merged(N, KIND, PK);
+  static constexpr bool M = chip_merged(sizeof(T), N, KIND);
   using FI = std::conditional_t<M, LineFFTM<N, +1, T>, LineFFT<N, +1, T>>;
   using FO = std::conditional_t<M, LineFFTM<N, -1, T>, LineFFT<N, -1, T>>;
   // consumes FI's output distribution

@@ -571,7 +571,7 @@ struct Upo2D {
       PSG_CUDA_TRY(cudaMemcpyAsync(plan.d_chip, ci.data(), sizeof(ChipInst<T>) * ci.size(),
                                    cudaMemcpyHostToDevice, stream));
       PSG_CUDA_TRY(chip2d_launch<T>(cp, plan.d_chip, (int)ci.size(),
-                                    chip_merged(n, kind, 0) ? plan.tw_merged : plan.tw, stream));
+                                    chip_merged(sizeof(T), n, kind) ? plan.tw_merged : plan.tw, stream));
       ++launches;
       if (is32)
         if (int rc = convert(out_jobs, false)) return rc;

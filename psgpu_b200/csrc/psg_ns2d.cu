@@ -310,7 +310,7 @@ struct Batch2D final : Batch2DBase {
           PSG_CUDA_TRY(cudaGetLastError());
         }
       } else PSG_CUDA_TRY(chip2d_launch<T>(plan_of(q, v), d_insts + off, count[q],
-                                           twiddles(q) + (chip_merged(16 << q, CHIP_STEP, (pk_mask >> q) & 1) ? 0 : kTables), s));
+                                           twiddles(q) + (chip_merged(sizeof(T), 16 << q, CHIP_STEP) ? 0 : kTables), s));
       if (present > 1) {
         PSG_CUDA_TRY(cudaEventRecord(ev_join[q], s));
         PSG_CUDA_TRY(cudaStreamWaitEvent(st, ev_join[q], 0));
