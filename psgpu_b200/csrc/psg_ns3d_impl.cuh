@@ -776,17 +776,17 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
     }
     T xi[E], et[E], zt[E], u[E], v[E], w[E];
     if constexpr (PK != 0) {
-      // packed: (u + i rho_x, v + i rho_y) -> (w + i rho_z, xi + i eta) -> zeta
+      // packed: (u + i v, rho_x + i rho_y) -> (w + i rho_z, xi + i eta) -> zeta
       // alone for the Boussinesq fields (u.grad rho first, so that at most six
-      // physical fields are live); (xi + i eta, zeta + i u) -> (v + i w) else
+      // physical fields are live; the two fields of a line share its rounding, so
+      // the velocities are kept from the density's gradients, but for w); (xi + i
+      // eta, zeta + i u) -> (v + i w) else
       if constexpr (BOUS) {
         T rx[E], ry[E], n4[E];
-        R::c2r_quad(src + 3 * fs, src + 6 * fs, src + 4 * fs, src + 7 * fs, K, gi,
-                                 s_tw, ex, u, rx, v, ry);
+        R::c2r_quad(src + 3 * fs, src + 4 * fs, src + 6 * fs, src + 7 * fs, K, gi, s_tw, ex, u, v, rx, ry);
 #pragma unroll
         for (int e = 0; e < E; ++e) n4[e] = u[e] * rx[e] + v[e] * ry[e];
-        R::c2r_quad(src + 5 * fs, src + 8 * fs, src, src + fs, K, gi, s_tw, ex, w, rx,
-                                 xi, et);
+        R::c2r_quad(src + 5 * fs, src + 8 * fs, src, src + fs, K, gi, s_tw, ex, w, rx, xi, et);
 #pragma unroll
         for (int e = 0; e < E; ++e) n4[e] = (n4[e] + w[e] * rx[e]) * hscale;
         R::c2r_pair(src + 2 * fs, nullptr, K, gi, s_tw, ex, zt, ry);
