@@ -140,8 +140,8 @@ __device__ __forceinline__ bool tile_wait(uint64_t* bar, int* s_ok, int* status)
 //
 // MODE 3 / 4 (linearised step): the 3-vectors of the adjoint's and the tangent's
 // cross products, z = in and x = in2 passed through spectral operators (OP_ID,
-// OP_CURL = i k x, OP_BS = i k x / k^2) and masked to the kept modes: z, C x,
-// B z (adjoint, nine fields) and z, B z, x, B x (tangent, twelve).
+// OP_CURL = i k x, OP_BS = i k x / k^2) and masked to the kept modes: z, B z,
+// C x (adjoint, nine fields) and z, B z, x, B x (tangent, twelve).
 // MODE 2 (scale): the fields of the Boussinesq adjoint's scalar products,
 // [psi, i k rho, B w] from psi = in2.c[0] and (w, rho) = in.c[0..3].
 // ---------------------------------------------------------------------------
@@ -276,8 +276,8 @@ pass_a(Geom3<T> g, Fields4<T> in, cpx<T>* __restrict__ out, const cpx<T>* __rest
         if (MODE >= 3) {
           if (tk > (T)0) {
             const int v3 = f / 3, comp = f % 3;  // which vector of the mode's list
-            const int sl = MODE == 3 ? (v3 == 1) : (v3 >= 2);
-            const int op = MODE == 3 ? (v3 == 0 ? OP_ID : v3 == 1 ? OP_CURL : OP_BS) : (v3 & 1) ? OP_BS : OP_ID;
+            const int sl = v3 >= 2;
+            const int op = (MODE == 3 && v3 == 2) ? OP_CURL : (v3 & 1) ? OP_BS : OP_ID;
             const cpx<T> x[3] = {s_in[(3 * sl) * Y * W + o], s_in[(3 * sl + 1) * Y * W + o],
                                  s_in[(3 * sl + 2) * Y * W + o]};
             r = spec_op<T>(op, comp, x, kx, ky, kz, tk);
@@ -709,22 +709,21 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
     const T hscale = (T)0.5 * scale;  // products of a paired forward transform
     if (NF == 7) {
       // scalar products of the Boussinesq adjoint: psi * (i k rho), psi * u
+      // (psi alone in its line, as the linearised fields below)
       T ps[E], ga[E], gb[E], p0[E], p1[E], p2[E];
-      R::c2r_pair(src, src + fs, K, gi, s_tw, ex, ps, ga);
-#pragma unroll
-      for (int e = 0; e < E; ++e) p0[e] = ps[e] * ga[e] * hscale;
-      R::c2r_pair(src + 2 * fs, src + 3 * fs, K, gi, s_tw, ex, ga, gb);
-#pragma unroll
-      for (int e = 0; e < E; ++e) { p1[e] = ps[e] * ga[e] * hscale; p2[e] = ps[e] * gb[e] * hscale; }
-      R::r2c_pair(p0, p1, K, XP, gi, two, ex, dst, dst + fstride, tstride);
-      R::c2r_pair(src + 4 * fs, src + 5 * fs, K, gi, s_tw, ex, ga, gb);
+      R::c2r_pair(src, nullptr, K, gi, s_tw, ex, ps, ga);
+      R::c2r_pair(src + fs, src + 2 * fs, K, gi, s_tw, ex, ga, gb);
 #pragma unroll
       for (int e = 0; e < E; ++e) { p0[e] = ps[e] * ga[e] * hscale; p1[e] = ps[e] * gb[e] * hscale; }
+      R::r2c_pair(p0, p1, K, XP, gi, two, ex, dst, dst + fstride, tstride);
+      R::c2r_pair(src + 3 * fs, src + 4 * fs, K, gi, s_tw, ex, ga, gb);
+#pragma unroll
+      for (int e = 0; e < E; ++e) { p2[e] = ps[e] * ga[e] * hscale; p0[e] = ps[e] * gb[e] * hscale; }
       R::r2c_pair(p2, p0, K, XP, gi, two, ex, dst + 2 * fstride, dst + 3 * fstride, tstride);
-      R::c2r_pair(src + 6 * fs, nullptr, K, gi, s_tw, ex, ga, gb);
+      R::c2r_pair(src + 5 * fs, src + 6 * fs, K, gi, s_tw, ex, ga, gb);
       release();
 #pragma unroll
-      for (int e = 0; e < E; ++e) p2[e] = ps[e] * ga[e] * hscale;
+      for (int e = 0; e < E; ++e) { p1[e] = ps[e] * ga[e] * hscale; p2[e] = ps[e] * gb[e] * hscale; }
       R::r2c_pair(p1, p2, K, XP, gi, two, ex, dst + 4 * fstride, dst + 5 * fstride, tstride);
       __syncwarp();
       continue;
@@ -741,29 +740,37 @@ pass_c(Geom3<T> g, const cpx<T>* __restrict__ in, cpx<T>* __restrict__ out,
             n[k][e] = add ? n[k][e] + x : x;
           }
       };
-      T a[3][E], b3[3][E], n[3][E];
-      R::c2r_pair(src + 3 * fs, src + 4 * fs, K, gi, s_tw, ex, b3[0], b3[1]);
+      // No line holds a field of z beside one of x: the fields of a line share its
+      // rounding, and x may be far the smaller (an adjoint step's is dt times the
+      // adjoint; with z_0 + i (C x)_2 a 64^3 FP32 gradient through 24 steps erred
+      // twice as far).
+      T a[3][E], b3[3][E], n[3][E], t[E];
       if constexpr (NF == 9 + kLinAdj) {
-        R::c2r_pair(src + 5 * fs, src, K, gi, s_tw, ex, b3[2], a[0]);
-        R::c2r_pair(src + fs, src + 2 * fs, K, gi, s_tw, ex, a[1], a[2]);
+        R::c2r_pair(src + 6 * fs, src + 7 * fs, K, gi, s_tw, ex, b3[0], b3[1]);
+        R::c2r_pair(src + 8 * fs, nullptr, K, gi, s_tw, ex, b3[2], t);
+        R::c2r_pair(src, src + fs, K, gi, s_tw, ex, a[0], a[1]);
+        R::c2r_pair(src + 2 * fs, src + 3 * fs, K, gi, s_tw, ex, a[2], t);
         cross(a, b3, n, hscale, false);  // -(z x Cx)
         R::r2c_pair(n[0], n[1], K, XP, gi, two, ex, dst, dst + fstride, tstride);
-        R::c2r_pair(src + 6 * fs, src + 7 * fs, K, gi, s_tw, ex, a[0], a[1]);
         T last[E];
 #pragma unroll
-        for (int e = 0; e < E; ++e) last[e] = n[2][e];
-        R::c2r_pair(src + 8 * fs, nullptr, K, gi, s_tw, ex, a[2], n[2]);
+        for (int e = 0; e < E; ++e) { last[e] = n[2][e]; a[0][e] = t[e]; }
+        R::c2r_pair(src + 4 * fs, src + 5 * fs, K, gi, s_tw, ex, a[1], a[2]);
         release();
         cross(b3, a, n, hscale, false);  // -(Cx x Bz)
         R::r2c_pair(last, n[0], K, XP, gi, two, ex, dst + 2 * fstride, dst + 3 * fstride, tstride);
         R::r2c_pair(n[1], n[2], K, XP, gi, two, ex, dst + 4 * fstride, dst + 5 * fstride, tstride);
       } else {
-        R::c2r_pair(src + 5 * fs, src + 6 * fs, K, gi, s_tw, ex, b3[2], a[0]);
-        R::c2r_pair(src + 7 * fs, src + 8 * fs, K, gi, s_tw, ex, a[1], a[2]);
+        T t2[E];
+        R::c2r_pair(src + 3 * fs, src + 4 * fs, K, gi, s_tw, ex, b3[0], b3[1]);
+        R::c2r_pair(src + 5 * fs, src, K, gi, s_tw, ex, b3[2], t);
+        R::c2r_pair(src + 6 * fs, src + 7 * fs, K, gi, s_tw, ex, a[0], a[1]);
+        R::c2r_pair(src + 8 * fs, src + 9 * fs, K, gi, s_tw, ex, a[2], t2);
         cross(b3, a, n, hscale, false);  // -(Bz x x)
-        R::c2r_pair(src + 9 * fs, src + 10 * fs, K, gi, s_tw, ex, a[0], a[1]);
-        R::c2r_pair(src + 11 * fs, src, K, gi, s_tw, ex, a[2], b3[0]);
+#pragma unroll
+        for (int e = 0; e < E; ++e) { b3[0][e] = t[e]; a[0][e] = t2[e]; }
         R::c2r_pair(src + fs, src + 2 * fs, K, gi, s_tw, ex, b3[1], b3[2]);
+        R::c2r_pair(src + 10 * fs, src + 11 * fs, K, gi, s_tw, ex, a[1], a[2]);
         release();
         cross(a, b3, n, hscale, true);  // -(Bx x z)
         R::r2c_pair(n[0], n[1], K, XP, gi, two, ex, dst, dst + fstride, tstride);

@@ -163,7 +163,7 @@ struct Plane {
     auto cross1 = [&](int a, int b) {
       return -(fld(a + k1, y, x) * fld(b + k2, y, x) - fld(a + k2, y, x) * fld(b + k1, y, x)) * sc;
     };
-    if constexpr (NF == 9 + kLinAdj) return o < 3 ? cross1(0, 3) : cross1(3, 6);
+    if constexpr (NF == 9 + kLinAdj) return o < 3 ? cross1(0, 6) : cross1(6, 3);
     else if constexpr (NF == 12 + kLinTan) return cross1(3, 6) + cross1(9, 0);
     else if (NF == 9 && o == 3)
       return (fld(3, y, x) * fld(6, y, x) + fld(4, y, x) * fld(7, y, x) + fld(5, y, x) * fld(8, y, x)) * sc;
@@ -235,27 +235,31 @@ struct Plane {
           forward(n[2], n4, 2, yg, live);
         }
       } else if constexpr (NF == 9 + kLinAdj) {
-        T last[E];
-        inverse(3, 4, y, b[0], b[1]);
-        inverse(5, 0, y, b[2], a[0]);
-        inverse(1, 2, y, a[1], a[2]);
+        // lines as in pass C: none holds a field of z beside one of x
+        T last[E], t[E];
+        inverse(6, 7, y, b[0], b[1]);
+        inverse(8, -1, y, b[2], t);
+        inverse(0, 1, y, a[0], a[1]);
+        inverse(2, 3, y, a[2], t);
         cross(a, b, n, h, false);  // -(z x Cx)
         forward(n[0], n[1], 0, yg, live);
 #pragma unroll
-        for (int e = 0; e < E; ++e) last[e] = n[2][e];
-        inverse(6, 7, y, a[0], a[1]);
-        inverse(8, -1, y, a[2], n[2]);
+        for (int e = 0; e < E; ++e) { last[e] = n[2][e]; a[0][e] = t[e]; }
+        inverse(4, 5, y, a[1], a[2]);
         cross(b, a, n, h, false);  // -(Cx x Bz)
         forward(last, n[0], 2, yg, live);
         forward(n[1], n[2], 4, yg, live);
       } else {
+        T t[E], t2[E];
         inverse(3, 4, y, b[0], b[1]);
-        inverse(5, 6, y, b[2], a[0]);
-        inverse(7, 8, y, a[1], a[2]);
+        inverse(5, 0, y, b[2], t);
+        inverse(6, 7, y, a[0], a[1]);
+        inverse(8, 9, y, a[2], t2);
         cross(b, a, n, h, false);  // -(Bz x x)
-        inverse(9, 10, y, a[0], a[1]);
-        inverse(11, 0, y, a[2], b[0]);
+#pragma unroll
+        for (int e = 0; e < E; ++e) { b[0][e] = t[e]; a[0][e] = t2[e]; }
         inverse(1, 2, y, b[1], b[2]);
+        inverse(10, 11, y, a[1], a[2]);
         cross(a, b, n, h, true);  // -(Bx x z)
 #pragma unroll
         for (int e = 0; e < E; ++e) n[2][e] *= (T)2;
