@@ -176,13 +176,16 @@ struct Batch2D final : Batch2DBase {
       const long nk = nkt2(sizes[i]);
       sums += global[size_class(sizes[i])] ? 4 * nk + 3L * sizes[i] * (sizes[i] / 3 + 1) : nk;
     }
-    // twiddle tables of every size: the merged transforms', then LineFFT's
+    // twiddle tables of every size: the merged transforms' (where a size present takes
+    // them: 80-bit sines, some 10 us a size), then LineFFT's
     const long twlen = 2 * kTables;
     PSG_CUDA_TRY(cudaMalloc(&pool, sizeof(cpx<T>) * (total + sums + twlen)));
     PSG_CUDA_TRY(cudaMemset(pool, 0, sizeof(cpx<T>) * (total + sums + twlen)));
     twp = pool + total + sums;
     std::vector<cpx<T>> h(twlen);
-    for (int q = 0; q < kClasses; ++q) chip_tables<T>(16 << q, h.data() + (twiddles(q) - twp));
+    for (int q = 0; q < kClasses; ++q)
+      if (count[q] && chip_merged(sizeof(T), 16 << q, CHIP_STEP))
+        chip_tables<T>(16 << q, h.data() + (twiddles(q) - twp));
     tables2d(h.data() + kTables);
     PSG_CUDA_TRY(cudaMemcpy(twp, h.data(), sizeof(cpx<T>) * twlen, cudaMemcpyHostToDevice));
     PSG_CUDA_TRY(cudaMalloc(&d_insts, sizeof(ChipInst<T>) * ninst));
