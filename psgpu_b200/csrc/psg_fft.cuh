@@ -206,8 +206,10 @@ struct LineFFT {
 // tau b), six multiply-adds as well, inherits the sum's rounding: 1.07 to 1.12 and
 // 0.98 to 1.18.)  Per 256-point line and lane: 340 FP instructions instead of 396; the
 // x-pass, bound by its arithmetic, went from 116 to 108 us (256^3 FP32), 229 to 188
-// (256^3 FP64) and 41 to 35 (128^3 FP64).  The 2D search's small grids, the
-// global-memory 2D kernels and the allocation-free step keep LineFFT.
+// (256^3 FP64) and 41 to 35 (128^3 FP64).  LineFFT stays with the 2D
+// integrator's FP32 steps, its tangent and 256^2, the search's small grids, the
+// global-memory 2D kernels and the allocation-free step: the tables' error, the same
+// at every right-hand side, is what the merged form has more of (psg_chip2d.cuh).
 // ---------------------------------------------------------------------------
 
 // a, b <- a + f b, a - f b with f = c (1 + i t)

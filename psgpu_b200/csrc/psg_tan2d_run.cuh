@@ -156,7 +156,7 @@ struct IntPlan {
     tw_merged = tw + 2 * n;
     std::vector<cpx<T>> h(4 * n);
     tan2d_tables<T>(n, h.data());
-    chip_tables<T>(n, h.data() + 2 * n);
+    if (chip_merged(sizeof(T), n, CHIP_BASE)) chip_tables<T>(n, h.data() + 2 * n);
     PSG_CUDA_TRY(cudaMemcpy(tw, h.data(), sizeof(cpx<T>) * 4 * n, cudaMemcpyHostToDevice));
     PSG_CUDA_TRY(cudaMalloc(&d_inst, (sizeof(InstTan2D<T>) + sizeof(ChipInst<T>)) * ng));
     d_chip = reinterpret_cast<ChipInst<T>*>(d_inst + ng);
